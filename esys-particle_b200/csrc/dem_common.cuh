@@ -72,12 +72,30 @@ __device__ __forceinline__ void for_neighbour_cells(const Grid& g, int c, const 
   }
 }
 
-// 32-byte read-only gather through the non-coherent (texture) path.  Only for
-// arrays the running kernel does not write (the step's input buffer).
+// 32-byte accesses (256-bit, sm_100).  Every double4 record lies at a multiple of 32 bytes: the
+// arrays are whole allocations or start at whole records of one.  A record is one sector, so one
+// access per lane halves the LSU's passes against two 16-byte ones.
+// Read-only gather through the non-coherent path: only for arrays the running kernel does not
+// write (the step's input buffer).
 __device__ __forceinline__ double4 ldg4(const double4* p) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-  return make_double4(a.x, a.y, b.x, b.y);
+  double4 r;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+// Two consecutive float4 that start at a multiple of 32 bytes, read-only.
+__device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+// Read at L2 (data that other SMs write while the kernel runs).
+__device__ __forceinline__ double4 ldcg4(const double4* p) {
+  double4 r;
+  asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p) : "memory");
+  return r;
+}
+__device__ __forceinline__ void st4(double4* p, const double4& v) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
 }
 
 // Bring a line into L1 without holding registers (records a kernel reads later).

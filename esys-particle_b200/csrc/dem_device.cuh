@@ -25,6 +25,8 @@ enum : int {
   CTRL_REBUILD = 1,     // some particle moved further than verletDist/2
   CTRL_BROKE = 2,       // at least one bond broke in the last force evaluation
   CTRL_OVERFLOW = 4,    // an event buffer overflowed
+  CTRL_LOST = 8,        // a grid barrier of the multi-step kernel gave up (its bounded wait ran out)
+  CTRL_FULL = 16,       // the multi-step kernel left before a step: a block's pruned entries do not fit it
 };
 
 constexpr int kMaxWalls = 8;
@@ -191,7 +193,41 @@ struct StepArgs {
   long long* step_counter;  // timesteps completed on the device
   int* ctrl;                // CTRL_* bits raised by this chunk of steps
   int* stop;                // set by the last block when ctrl != 0: later steps of the chunk skip
+  unsigned long long* run_word;  // multi-step kernel: the two words of its grid barrier, zero at launch
 };
+
+// Launch of the multi-step kernel (dem_run.cuh).
+constexpr int kRunThreads = 512;
+struct RunArgs {
+  int nsteps;     // timesteps of this launch
+  int blocks;     // at most one per SM
+  int chunk;      // consecutive slots dealt to a block at a time
+  int ppb;        // particles per block: chunk x rounds
+  int one;        // 1: a block keeps its particles' records in shared memory
+  int pool;       // pruned entries a block can hold, at most 65535
+  int room;       // entries whose results it can hold at a time
+  float half;     // least allowance of movement of the first prune
+  float horizon;  // steps whose movement at the particle's speed its allowance covers
+};
+// Shared memory of one of its blocks: byte offsets of the arrays and the total.
+struct RunLayout {
+  size_t coef, res, entry, limit, at, owner, bytes;
+};
+__host__ __device__ inline RunLayout run_layout(bool rot, bool fric, bool moment, bool fp32, bool one, int ppb, int pool,
+                                                int room) {
+  RunLayout L;
+  size_t o = one ? (size_t)8 * (rot ? 21 : 12) * ppb : 0;
+  auto take = [&](size_t bytes) { const size_t at = o; o = (o + bytes + 15) & ~(size_t)15; return at; };
+  o = (o + 15) & ~(size_t)15;
+  L.coef = take((size_t)24 * pool);
+  L.res = take((size_t)(fp32 ? 4 : 8) * (moment ? 9 : (fric ? 6 : 3)) * room);
+  L.entry = take((size_t)8 * pool);
+  L.limit = take((size_t)12 * ppb);
+  L.at = take((size_t)2 * (ppb + 1));
+  L.owner = take((size_t)2 * pool);
+  L.bytes = o;
+  return L;
+}
 
 // Batched ensemble step (dem_batch.cuh): the specimens' step arguments in a device table.
 struct BatchArgs {

@@ -62,6 +62,11 @@ void launch_step(const StepArgs& a, bool rot, int tpp, bool split, cudaStream_t 
 void launch_bond_pass_f64(const StepArgs& a, bool eval, cudaStream_t s);
 void launch_step_fp32(const StepArgs& a, bool rot, int tpp, bool eval, bool split, cudaStream_t s);
 
+// Up to ra.nsteps timesteps in one cooperative launch (dem_run.cuh), from the step the device counter
+// stands at; a.cur is the input buffer of the first.
+cudaError_t launch_run(const StepArgs& a, bool rot, const RunArgs& ra, cudaStream_t s);
+cudaError_t launch_run_fp32(const StepArgs& a, bool rot, const RunArgs& ra, cudaStream_t s);
+
 // batched ensemble (dem_batch.cu, dem_batch_fp32.cu)
 void launch_batch_step(const BatchArgs& B, bool rot, bool el, bool fr, bool bd, bool gather, int tpp, cudaStream_t s);
 void launch_batch_step_fp32(const BatchArgs& B, bool rot, bool el, bool fr, bool bd, bool gather, int tpp,

@@ -72,12 +72,13 @@ struct FricOutT {
 };
 using FricOut = FricOutT<double>;
 
-// CRotFrictionInteraction::calcSimpleForces (Model/RotFricInteraction.cpp:171-231).
+// CRotFrictionInteraction::calcSimpleForces (Model/RotFricInteraction.cpp:171-231).  part = r2 / (r1 + r2),
+// which places the contact point, is a constant of the pair.
 template <class S>
-__device__ __forceinline__ void law_friction_t(S k_eff, S ks_eff, double mu_s, double mu_d, double dt,
-                                               const V3<S>& x1, double r1, const V3<S>& v1, const V3<S>& w1,
-                                               const V3<S>& x2, double r2, const V3<S>& v2, const V3<S>& w2,
-                                               V3<S> Ffric, bool slipping, FricOutT<S>& o) {
+__device__ __forceinline__ void law_friction_at(S k_eff, S ks_eff, double part, double mu_s, double mu_d, double dt,
+                                                const V3<S>& x1, double r1, const V3<S>& v1, const V3<S>& w1,
+                                                const V3<S>& x2, double r2, const V3<S>& v2, const V3<S>& w2,
+                                                V3<S> Ffric, bool slipping, FricOutT<S>& o) {
   using VS = V3<S>;
   double mu_current = slipping ? mu_d : mu_s;
   const VS D = x1 - x2;
@@ -86,7 +87,7 @@ __device__ __forceinline__ void law_friction_t(S k_eff, S ks_eff, double mu_s, d
   if (dist < (eq_dist * eq_dist)) {
     dist = sqrt(dist);
     const VS force = D * (k_eff * (dist - eq_dist) / dist);
-    const VS pos = x2 + (r2 / eq_dist) * D;
+    const VS pos = x2 + part * D;
     const VS vp1 = v1 + cross(w1, pos - x1);
     const VS vp2 = v2 + cross(w2, pos - x2);
     VS ds = (vp2 - vp1) * dt;
@@ -112,6 +113,13 @@ __device__ __forceinline__ void law_friction_t(S k_eff, S ks_eff, double mu_s, d
     o.slipping = false;
     o.touching = false;
   }
+}
+template <class S>
+__device__ __forceinline__ void law_friction_t(S k_eff, S ks_eff, double mu_s, double mu_d, double dt,
+                                               const V3<S>& x1, double r1, const V3<S>& v1, const V3<S>& w1,
+                                               const V3<S>& x2, double r2, const V3<S>& v2, const V3<S>& w2,
+                                               const V3<S>& Ffric, bool slipping, FricOutT<S>& o) {
+  law_friction_at<S>(k_eff, ks_eff, r2 / (r1 + r2), mu_s, mu_d, dt, x1, r1, v1, w1, x2, r2, v2, w2, Ffric, slipping, o);
 }
 __device__ __forceinline__ void law_friction(double k_eff, double ks_eff, double mu_s, double mu_d, double dt,
                                              const V& x1, double r1, const V& v1, const V& w1, const V& x2, double r2,

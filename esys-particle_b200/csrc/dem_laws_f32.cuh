@@ -45,10 +45,11 @@ struct FricOutF {
 };
 
 // CRotFrictionInteraction::calcSimpleForces in the FP32 form.  D = x1 - x2 (FP64);
-// v, w are the FP32 copies of the particles' velocities and spins.
-__device__ __forceinline__ void law_friction_f32(double k_eff, double ks_eff, double mu_s, double mu_d, float dt,
-                                                 const V& D, double r1, double r2, const Vf& v1, const Vf& w1,
-                                                 const Vf& v2, const Vf& w2, Vf Ff, bool slipping, FricOutF& o) {
+// v, w are the FP32 copies of the particles' velocities and spins; part = r2 / (r1 + r2).
+__device__ __forceinline__ void law_friction_f32_at(double k_eff, double ks_eff, double part, double mu_s, double mu_d,
+                                                    float dt, const V& D, double r1, double r2, const Vf& v1,
+                                                    const Vf& w1, const Vf& v2, const Vf& w2, Vf Ff, bool slipping,
+                                                    FricOutF& o) {
   const double dist2 = dot(D, D);
   const double eq_dist = r1 + r2;
   if (dist2 < eq_dist * eq_dist) {
@@ -57,7 +58,7 @@ __device__ __forceinline__ void law_friction_f32(double k_eff, double ks_eff, do
     const Vf Df = cvt<float>(D);
     const Vf force = Df * (float)(k_eff * over / dist);
     // contact point x2 + r2/(r1+r2) D, as lever arms from each centre
-    const float a2 = (float)(r2 / eq_dist);
+    const float a2 = (float)part;
     const Vf arm2 = Df * a2;
     const Vf arm1 = arm2 - Df;
     const Vf vp1 = v1 + cross(w1, arm1);
@@ -90,6 +91,13 @@ __device__ __forceinline__ void law_friction_f32(double k_eff, double ks_eff, do
     o.slipping = false;
     o.touching = false;
   }
+}
+
+__device__ __forceinline__ void law_friction_f32(double k_eff, double ks_eff, double mu_s, double mu_d, float dt,
+                                                 const V& D, double r1, double r2, const Vf& v1, const Vf& w1,
+                                                 const Vf& v2, const Vf& w2, const Vf& Ff, bool slipping,
+                                                 FricOutF& o) {
+  law_friction_f32_at(k_eff, ks_eff, r2 / (r1 + r2), mu_s, mu_d, dt, D, r1, r2, v1, w1, v2, w2, Ff, slipping, o);
 }
 
 }  // namespace dem

@@ -130,7 +130,13 @@ struct DemSim {
   Grid g{};
   cudaStream_t s = nullptr;
   int tpp = 0;           // 0 = choose from the mean adjacency length
-  int chunk = 64;        // steps launched per host round trip
+  int chunk = 0;         // steps launched per host round trip ("chunk"); 0 = kChunk, or kRunChunk in one multi-step launch
+  static constexpr int kChunk = 64, kRunChunk = 1024;
+  static constexpr int kRunMin = 4;        // multi-step kernel without resident records: fewer steps go out singly
+  static constexpr int kRunEntries = 256;  // list entries per block that a small specimen's block count aims at
+  // The multi-step kernel stays off until this neighbour search (counted by timestamp) after a launch
+  // whose pruned lists did not fit; searches it is off for double while that goes on.
+  int run_off_until = -1, run_backoff = 1;
   int store_forces = 1;
   int fp32 = 0;          // 1 = FP32-force / FP64-integration form
   int split = -1;        // -1 automatic, 0 fused step kernel, 1 pair kernel + integration kernel
@@ -170,8 +176,13 @@ struct DemSim {
   std::vector<double> wall_vel;  // per wall name, keyed by wig order at upload
   std::map<std::string, std::vector<double>> wall_loader;  // wall name -> velocity
   DBuf<unsigned> d_block_counter;
-  DBuf<long long> d_step;
-  DBuf<int> d_ctrl, d_stop;
+  // Device control words, in one block so that a chunk of steps is prepared by one memset and
+  // read back by one copy: the step counter, CTRL_* bits and stop word, the multi-step kernel's words.
+  DBuf<long long> d_ctl;
+  long long* d_step = nullptr;
+  int *d_ctrl = nullptr, *d_stop = nullptr;
+  unsigned long long* d_run = nullptr;
+  int num_sms = 0;       // of the current device; 0 until asked for
   int* h_ctrl = nullptr;  // pinned
   long long t = 0;
   int timestamp = 0, last_ns = -1;
@@ -193,11 +204,14 @@ struct DemSim {
   DemSim() {
     DEM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     DEM_CUDA(cudaMallocHost(&h_ctrl, 4 * sizeof(long long)));
-    d_block_counter.reserve(1); d_step.reserve(1); d_ctrl.reserve(1); d_stop.reserve(1); scalars.reserve(8);
+    d_block_counter.reserve(1); d_ctl.reserve(4); scalars.reserve(8);
+    d_step = d_ctl.p;
+    d_ctrl = reinterpret_cast<int*>(d_ctl.p + 1);
+    d_stop = d_ctrl + 1;
+    d_run = reinterpret_cast<unsigned long long*>(d_ctl.p + 2);
     DEM_CUDA(cudaMemsetAsync(d_block_counter.p, 0, sizeof(unsigned), s));
-    DEM_CUDA(cudaMemsetAsync(d_step.p, 0, sizeof(long long), s));
-    DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
-    DEM_CUDA(cudaMemsetAsync(d_stop.p, 0, sizeof(int), s));
+    DEM_CUDA(cudaMemsetAsync(d_step, 0, sizeof(long long), s));
+    clear_control();
     d_wall_force.reserve(kMaxWalls * 3);
     DEM_CUDA(cudaMemsetAsync(d_wall_force.p, 0, sizeof(double) * kMaxWalls * 3, s));
   }
@@ -213,7 +227,7 @@ struct DemSim {
     cell_count.release(); cell_start.release(); cell_cursor.release(); cell_list.release();
     scratch_i.release(); scratch_j.release(); scalars.release(); scan_tmp.release();
     d_walls.release(); d_wall_vel.release(); d_wall_partial.release(); d_wall_force.release();
-    d_block_counter.release(); d_step.release(); d_ctrl.release(); d_stop.release();
+    d_block_counter.release(); d_ctl.release();
     stage.release(); stage_slot.release(); scratch_d.release(); sig.release(); d_servo_idx.release(); d_brk.release(); rows.release(); pack_id.release();
     pack.release();
     if (h_ctrl) cudaFreeHost(h_ctrl);
@@ -223,6 +237,8 @@ struct DemSim {
   }
 
   void sync() { DEM_CUDA(cudaStreamSynchronize(s)); }
+  // The control bits, the stop word and the multi-step kernel's words, before a chunk of steps.
+  void clear_control() { DEM_CUDA(cudaMemsetAsync(d_ctl.p + 1, 0, 3 * sizeof(long long), s)); }
   // Capacity of a bonded group's failure-event log: every bond can fail once, so the
   // default never overflows; the "event_capacity" option sets a fixed size instead.
   int ev_cap = 0;
@@ -428,10 +444,7 @@ struct DemSim {
     launch_sync_vw(P, cur, s);
     StepArgs ea = make_args(cur);
     launch_step_fp32(ea, rot != 0, t_pp, true, false, s);
-    const int keep = chunk;
-    chunk = 1;
     step(1);
-    chunk = keep;
     std::vector<double4> f(n), fe(n), m(n), me(n);
     std::vector<unsigned> pf(n);
     DEM_CUDA(cudaMemcpyAsync(f.data(), P.force, sizeof(double4) * n, cudaMemcpyDeviceToHost, s));
@@ -498,9 +511,9 @@ struct DemSim {
     launch_set_state(P, cur, cnt, slots, pos ? d : nullptr, vel ? d + c3 : nullptr,
                      (angvel && rot) ? d + 2 * c3 : nullptr, (quat && rot) ? d + 3 * c3 : nullptr, s);
     // moved particles are checked like any displacement before the next step
-    launch_check_disp(P, cur, (0.5 * alpha) * (0.5 * alpha), d_ctrl.p, s);
-    pending_ctrl |= read_int(d_ctrl.p);
-    DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
+    launch_check_disp(P, cur, (0.5 * alpha) * (0.5 * alpha), d_ctrl, s);
+    pending_ctrl |= read_int(d_ctrl);
+    DEM_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(int), s));
     c_launches += 2;
     return 0;
   }
@@ -886,9 +899,10 @@ struct DemSim {
     a.wall_partial = d_wall_partial.p;
     a.wall_force = d_wall_force.p;
     a.block_counter = d_block_counter.p;
-    a.step_counter = d_step.p;
-    a.ctrl = d_ctrl.p;
-    a.stop = d_stop.p;
+    a.step_counter = d_step;
+    a.ctrl = d_ctrl;
+    a.stop = d_stop;
+    a.run_word = d_run;
     return a;
   }
 
@@ -899,24 +913,68 @@ struct DemSim {
     return bond.empty() || bond_pass || fp32;
   }
 
-  // Lanes per particle when none is set.  A specimen with at least as many particles as the
-  // GPU keeps step threads resident (3 blocks of 256 per SM) already fills it at one lane per
-  // particle, which measured fastest on the 250k shear cell and the 1M bonded block; a smaller
-  // one spreads each particle's adjacency over lanes by its mean length.  The tiled kernels
-  // (kTiled) are chosen explicitly or by the ensemble autotuner.
+  int sms() {
+    if (!num_sms) {
+      int dev = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+      if (num_sms <= 0) num_sms = 148;
+    }
+    return num_sms;
+  }
+
+  // The multi-step kernel's launch (dem_run.cuh); false where dem_step takes single-step launches:
+  // with bonds, the lane, tiled and warp-cooperative forms chosen by the caller, a specimen whose
+  // particles alone fill a block's shared memory, or one whose pruned lists did not fit lately.
+  bool run_shape(RunArgs& ra) {
+    if (!bond.empty() || split == 1 || tpp > 1 || n < 1 || timestamp < run_off_until) return false;
+    bool fric = false, moment = false;
+    long long m2 = 0;
+    for (auto& d : dyn) {
+      fric = fric || d.second.kind != 0;
+      moment = moment || (rot && d.second.kind != 0);
+      m2 += 2LL * d.second.m;
+    }
+    const double mean = (double)m2 / n;
+    // one block per SM; a small specimen takes fewer blocks, of kRunEntries entries or so
+    const double want = n * std::max(mean, 1.0) / kRunEntries;
+    ra.blocks = (int)std::min<double>(sms(), std::max(1.0, std::ceil(want)));
+    ra.chunk = n >= 256LL * ra.blocks ? 32 : (n >= 8LL * ra.blocks ? 8 : 1);
+    const int groups = (n + ra.chunk - 1) / ra.chunk;
+    ra.ppb = ra.chunk * ((groups + ra.blocks - 1) / ra.blocks);
+    ra.half = (float)(alpha / 16);
+    ra.horizon = 64.f;
+    constexpr size_t kSmem = 220 * 1024;  // of a block's 227 KB, less the kernel's static arrays
+    // every entry of the list in shared memory, results included, beside the particles' records
+    const long long worst = std::max(64LL, (long long)std::ceil(1.25 * mean * ra.ppb));
+    ra.one = 1;
+    if (worst < 65536) {
+      ra.pool = ra.room = (int)worst;
+      if (run_layout(rot, fric, moment, fp32, true, ra.ppb, ra.pool, ra.room).bytes <= kSmem) return true;
+    }
+    // else the records stay in L2, and what is left is shared 60:40 between entries and results
+    ra.one = 0;
+    const size_t fixed = run_layout(rot, fric, moment, fp32, false, ra.ppb, 0, 0).bytes + 128;
+    if (ra.ppb > 65535 || fixed > kSmem / 2) return false;
+    const size_t left = kSmem - fixed, res = (size_t)(fp32 ? 4 : 8) * (moment ? 9 : (fric ? 6 : 3));
+    ra.pool = (int)std::min<size_t>(std::min<long long>(worst, 65535), left * 6 / 10 / 34);
+    ra.room = (int)std::min<size_t>(ra.pool, (left - (size_t)34 * ra.pool) / res);
+    return ra.room >= 1024 && ra.pool >= ra.ppb / 4;
+  }
+
+  // Lanes per particle of the single-step kernels when none is set.  Without bonds one lane: the
+  // multi-step kernel's order of summation, whichever of the two takes a call.  With bonds, a
+  // specimen with at least as many particles as the GPU keeps step threads resident (3 blocks of
+  // 256 per SM) already fills it at one lane per particle, and a smaller one spreads each
+  // particle's adjacency over lanes by its mean length.  The tiled kernels (kTiled) are chosen
+  // explicitly or by the ensemble autotuner.
   int pick_tpp() {
     if (tpp) return tpp == kTiled && !tiled_ok() ? 1 : tpp;
-    static const long long resident = [] {
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      return 768LL * (sms > 0 ? sms : 148);
-    }();
-    if (n >= resident) return 1;
+    if (bond.empty() || n >= 768LL * sms()) return 1;
     long long e = 0;
     for (auto& d : dyn) e += 2LL * d.second.m;
     for (auto& b : bond) e += 2LL * b.second.nb;
-    double mean = n ? (double)e / n : 0.0;
+    const double mean = n ? (double)e / n : 0.0;
     if (mean >= 12) return 8;
     if (mean >= 6) return 4;
     if (mean >= 2.5) return 2;
@@ -953,12 +1011,14 @@ struct DemSim {
     while (done < nsteps) {
       if (!prepare()) return -2;
       // launch a chunk of force + integration steps
-      const int k = std::min(chunk, nsteps - done);
       const int t_pp = pick_tpp();
-      const int grid = step_grid(n, t_pp);
+      RunArgs ra{};
+      const bool multi = run_shape(ra) && (ra.one || nsteps - done >= kRunMin);
+      const int k = std::min(multi ? std::min(chunk > 0 ? chunk : kRunChunk, kRunChunk) : (chunk > 0 ? chunk : kChunk),
+                             nsteps - done);
+      const int grid = std::max(step_grid(n, t_pp), sms());  // partials of either kernel's blocks
       d_wall_partial.reserve((size_t)grid * kMaxWalls * 3);
-      DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
-      DEM_CUDA(cudaMemsetAsync(d_stop.p, 0, sizeof(int), s));
+      clear_control();
       const long long t0 = t;
       const long long cps = contacts_per_step();
       if (profile) {
@@ -967,23 +1027,41 @@ struct DemSim {
       }
       if (fp32 && t_pp == kTiled) launch_sync_vw(P, cur, s);  // only the tiled kernels read the shadow
       const bool two = split == 1;  // automatic = fused: measured faster on the 250k shear cell
-      for (int j = 0; j < k; ++j) {
-        StepArgs a = make_args((cur + j) & 1);
+      if (multi) {
+        StepArgs a = make_args(cur);
         a.force_step = t_last;
-        a.skip_vw = t_pp != kTiled;  // only the tiled kernels read the FP32 velocity shadow
-        if (fp32) launch_step_fp32(a, rot != 0, t_pp, false, two, s);
-        else launch_step(a, rot != 0, t_pp, two, s);
+        ra.nsteps = k;
+        DEM_CUDA(fp32 ? launch_run_fp32(a, rot != 0, ra, s) : launch_run(a, rot != 0, ra, s));
+      } else {
+        for (int j = 0; j < k; ++j) {
+          StepArgs a = make_args((cur + j) & 1);
+          a.force_step = t_last;
+          a.skip_vw = t_pp != kTiled;  // only the tiled kernels read the FP32 velocity shadow
+          if (fp32) launch_step_fp32(a, rot != 0, t_pp, false, two, s);
+          else launch_step(a, rot != 0, t_pp, two, s);
+        }
+        DEM_CUDA(cudaGetLastError());
       }
-      DEM_CUDA(cudaGetLastError());
       if (profile) DEM_CUDA(cudaEventRecord(ev1, s));
-      c_launches += two ? 2LL * k : k;
-      DEM_CUDA(cudaMemcpyAsync(h_ctrl, d_step.p, sizeof(long long), cudaMemcpyDeviceToHost, s));
-      DEM_CUDA(cudaMemcpyAsync(h_ctrl + 2, d_ctrl.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+      c_launches += multi ? 1 : (two ? 2LL * k : k);
+      DEM_CUDA(cudaMemcpyAsync(h_ctrl, d_ctl.p, 2 * sizeof(long long), cudaMemcpyDeviceToHost, s));  // counter, bits
       sync();
       long long dev_t;
       std::memcpy(&dev_t, h_ctrl, sizeof(long long));
       const int ran = (int)(dev_t - t0);
       pending_ctrl = h_ctrl[2];
+      if (pending_ctrl & CTRL_LOST) {
+        err = "a grid barrier of the multi-step kernel timed out";
+        return -3;
+      }
+      if (pending_ctrl & CTRL_FULL) {
+        run_off_until = timestamp + run_backoff;
+        run_backoff = std::min(64, 2 * run_backoff);
+        pending_ctrl &= ~CTRL_FULL;
+        if (ran == 0) continue;
+      } else if (multi) {
+        run_backoff = 1;
+      }
       overflowed |= take_overflow();
       // a BrittleBeamSC failure at the head of the chunk's first step stops it before any step
       if (ran < 0 || ran > k || (ran == 0 && !(pending_ctrl & CTRL_BROKE))) {
@@ -1184,8 +1262,7 @@ struct DemSim {
     for (int c = 0; c < win.nseg; ++c) {
       const int len = std::min(win.K, win.T - c * win.K);
       win_checkpoint(c);
-      DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
-      DEM_CUDA(cudaMemsetAsync(d_stop.p, 0, sizeof(int), s));
+      clear_control();
       for (int j = 0; j < len; ++j) {
         StepArgs a = make_args((cur + j) & 1);
         a.wall_hist = win.R.p;
@@ -1195,8 +1272,7 @@ struct DemSim {
       }
       DEM_CUDA(cudaGetLastError());
       c_launches += two ? 2LL * len : len;
-      DEM_CUDA(cudaMemcpyAsync(h_ctrl, d_step.p, sizeof(long long), cudaMemcpyDeviceToHost, s));
-      DEM_CUDA(cudaMemcpyAsync(h_ctrl + 2, d_ctrl.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+      DEM_CUDA(cudaMemcpyAsync(h_ctrl, d_ctl.p, 2 * sizeof(long long), cudaMemcpyDeviceToHost, s));  // counter, bits
       sync();
       long long dev_t;
       std::memcpy(&dev_t, h_ctrl, sizeof(long long));
@@ -1336,9 +1412,8 @@ struct DemSim {
       DEM_CUDA(cudaMemcpyAsync(d_brk.p, win.ck_brk.p + 2 * c, 2 * sizeof(int), cudaMemcpyDeviceToDevice, s));
     }
     win.tcv = win.t0 + (long long)c * win.K;
-    DEM_CUDA(cudaMemcpyAsync(d_step.p, &win.tcv, sizeof(long long), cudaMemcpyHostToDevice, s));
-    DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
-    DEM_CUDA(cudaMemsetAsync(d_stop.p, 0, sizeof(int), s));
+    DEM_CUDA(cudaMemcpyAsync(d_step, &win.tcv, sizeof(long long), cudaMemcpyHostToDevice, s));
+    clear_control();
   }
 
   // Step arguments of recomputed step j of a segment: state j -> j + 1 in the recompute
@@ -1438,9 +1513,8 @@ struct DemSim {
     }
     if (nw) DEM_CUDA(cudaMemcpyAsync(d_walls.p, win.save_walls.p, sizeof(WallDev) * nw, cudaMemcpyDeviceToDevice, s));
     DEM_CUDA(cudaMemcpyAsync(d_wall_force.p, win.save_wf.p, sizeof(double) * kMaxWalls * 3, cudaMemcpyDeviceToDevice, s));
-    DEM_CUDA(cudaMemcpyAsync(d_step.p, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
-    DEM_CUDA(cudaMemsetAsync(d_ctrl.p, 0, sizeof(int), s));
-    DEM_CUDA(cudaMemsetAsync(d_stop.p, 0, sizeof(int), s));
+    DEM_CUDA(cudaMemcpyAsync(d_step, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
+    clear_control();
     std::vector<double> acc(off);
     std::vector<double4> lh((size_t)4 * n);
     std::vector<unsigned> pf(n);
@@ -1966,7 +2040,7 @@ struct DemSim {
     // CLatticeMaster::loadCheckPointData (Parallel/LatticeMaster.cpp:780-820): the step counter,
     // then searchNeighbors(true) and updateInteractions
     t = timestep;
-    DEM_CUDA(cudaMemcpyAsync(d_step.p, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
+    DEM_CUDA(cudaMemcpyAsync(d_step, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
     sync();
     search_neighbors();
     resize_adjacency();
@@ -2033,7 +2107,7 @@ struct DemSim {
       DEM_CUDA(cudaMemcpyAsync(d_brk.p, win.ck_brk.p, 2 * sizeof(int), cudaMemcpyDeviceToDevice, s));
     }
     t = win.t0;
-    DEM_CUDA(cudaMemcpyAsync(d_step.p, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
+    DEM_CUDA(cudaMemcpyAsync(d_step, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
     pending_ctrl = 0;
     sync();
     if (win.brk) refresh_counts();
@@ -3130,8 +3204,8 @@ int dem_move_tagged(dem_sim* h, int tag, int mask, const double* d) {
   return guard(h, [&](DemSim& s) {
     dem::launch_move_tagged(s.P, s.cur, tag, d, s.s);
     // a host-side move is checked like any displacement (checkNeighbors runs after pre-runnables)
-    dem::launch_check_disp(s.P, s.cur, (0.5 * s.alpha) * (0.5 * s.alpha), s.d_ctrl.p, s.s);
-    s.pending_ctrl |= s.read_int(s.d_ctrl.p);
+    dem::launch_check_disp(s.P, s.cur, (0.5 * s.alpha) * (0.5 * s.alpha), s.d_ctrl, s.s);
+    s.pending_ctrl |= s.read_int(s.d_ctrl);
     return DEM_OK;
   });
 }

@@ -135,6 +135,170 @@ __device__ __forceinline__ void stress_add(double* S, const V& f, const V& pos, 
     for (int q = 0; q < 3; ++q) S[3 * p + q] -= fv[p] * rv[q];
 }
 
+// The partner's records and the pair's history through the read-only path (buffers that the
+// running kernel does not write).
+struct PairGather {
+  const ParticleBuf& in;
+  const DynDev& G;
+  int j, k;
+  __device__ __forceinline__ double4 v() const { return ldg4(in.vm + j); }
+  __device__ __forceinline__ double4 w() const { return ldg4(in.wi + j); }
+  __device__ __forceinline__ double4 h() const { return ldg4(G.hist_in + k); }
+  __device__ __forceinline__ float4 h32() const { return __ldg(G.hist32_in + k); }
+};
+
+// One dynamic-group pair seen from particle i (position and radius p4, velocity and spin v4, w4 or
+// their FP32 roundings vself, wself): its contribution to i's sums, and the pair's history when i
+// is the pair's p1 (lower id).  j the partner's slot, k the pair's index, pj the partner's
+// position record.  Contact is tested first from the positions alone; `late` gives the partner's
+// velocity / spin and the pair's history of a touching pair (a non-touching RotFriction pair just
+// resets its history).
+template <bool ROT, int FEAT, bool FP32, bool EVAL, class Late>
+__device__ __forceinline__ void pair_entry(const Grid& g, const DynDev& G, int k, bool isp1, const double4& p4,
+                                           const double4& pj, const double4& v4, const double4& w4, const Vf& vself,
+                                           const Vf& wself, double4* hist_out, float4* hist32_out, const Late& late,
+                                           V& Fp, V& Mp, KSum3& Fk, KSum3& Mk, double& Gs, double* stress) {
+  constexpr bool STRESS = !FP32 && (FEAT & F_STRESS) != 0;
+  // canonical orientation: p1 = lower id
+  const double4 pa = isp1 ? p4 : pj, pb = isp1 ? pj : p4;
+  const V x1 = xyz(pa), x2 = image_of(g, x1, xyz(pb));
+  const V D = x1 - x2;
+  const double eq_dist = pa.w + pb.w;
+  const bool touching = dot(D, D) < (eq_dist * eq_dist);  // the laws' contact test
+  if (G.kind == 0) {
+    if constexpr ((FEAT & F_ELASTIC) != 0) {
+      if (!touching) return;
+      if constexpr (!FP32) {
+        V f;
+        if (law_elastic(elastic_k(G.k, G.scaling, pa.w, pb.w), x1, pa.w, x2, pb.w, f)) {
+          if (isp1) Fp += -1.0 * f; else Fp += f;
+          if constexpr (STRESS) {  // CElasticInteraction::calcForces: at x2 + r2 / (r1 + r2) D
+            const V pos = x2 + (pb.w / eq_dist) * D;
+            stress_add(stress, isp1 ? -1.0 * f : f, pos, isp1 ? x1 : x2);
+          }
+        }
+      } else {
+        Vf f;
+        if (law_elastic_f32(elastic_k(G.k, G.scaling, pa.w, pb.w), D, pa.w, pb.w, f)) {
+          Fk.add(isp1 ? -f : f);
+          if (EVAL) Gs += (double)norm(f);
+        }
+      }
+    }
+  } else if (G.kind >= 2) {
+    // NRotFriction (CFrictionInteraction::calcForces) or HertzMindlin
+    // (CHertzMindlinInteraction::calcForces): forces only, history of the tangential force
+    if constexpr (!FP32 && (FEAT & F_NFRIC) != 0) {
+      if (!touching) {
+        if (isp1 && !EVAL) hist_out[k] = make_double4(0.0, 0.0, 0.0, 0.0);
+        return;
+      }
+      const double4 vj = late.v();
+      const double4 va = isp1 ? v4 : vj, vb = isp1 ? vj : v4;
+      const double4 h = late.h();
+      FricOut o;
+      if (G.kind == 2) {
+        double keff, kseff;
+        nfriction_k(G.k, G.ks, G.scaling, pa.w, pb.w, keff, kseff);
+        law_nfriction(keff, kseff, G.mu_s, G.dt, x1, pa.w, xyz(va), x2, pb.w, xyz(vb), mk(h.x, h.y, h.z), o);
+      } else if (G.kind == 3) {  // E in k, nu in ks; the normal force on p1 is +fn: negated for the common form
+        law_hertz_mindlin(G.k, G.ks, G.mu_s, G.dt, x1, pa.w, xyz(va), x2, pb.w, xyz(vb), mk(h.x, h.y, h.z), o);
+        o.fn = -1.0 * o.fn;
+      } else {  // HertzMindlinVisco: E, nu, mu, restitution in k, ks, mu_s, mu_d; masses in the w's
+        law_hertz_mindlin_visco(G.k, G.ks, G.mu_s, G.mu_d, G.dt, x1, pa.w, va.w, xyz(va), x2, pb.w, vb.w, xyz(vb),
+                                o);
+        o.fn = -1.0 * o.fn;
+      }
+      if constexpr (STRESS) {
+        const V pos = x2 + (pb.w / eq_dist) * D;
+        const V xs = isp1 ? x1 : x2;
+        stress_add(stress, isp1 ? -1.0 * o.fn : o.fn, pos, xs);
+        stress_add(stress, isp1 ? o.Ffric : -1.0 * o.Ffric, pos, xs);
+      }
+      if (isp1) {  // p1: -force, then +Ffric; p2: +force, then -Ffric
+        Fp += -1.0 * o.fn;
+        Fp += o.Ffric;
+        if (!EVAL)
+          hist_out[k] = make_double4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
+                                     (o.slipping ? 1.0 : 0.0) + (o.touching ? 2.0 : 0.0));
+      } else {
+        Fp += o.fn;
+        Fp += -1.0 * o.Ffric;
+      }
+      if (EVAL) Gs += norm(o.fn) + norm(o.Ffric);
+    }
+  } else {
+    if constexpr (ROT && (FEAT & F_FRIC) != 0) {
+      if (!touching) {  // CRotFrictionInteraction::calcSimpleForces, no-contact branch
+        if (isp1 && !EVAL) {
+          if (FP32) hist32_out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          else hist_out[k] = make_double4(0.0, 0.0, 0.0, 0.0);
+        }
+        return;
+      }
+      double keff, kseff;
+      friction_k(G.k, G.ks, G.scaling, G.meanR, pa.w, pb.w, keff, kseff);
+      if constexpr (!FP32) {
+        const double4 vj = late.v(), wj = late.w();
+        const double4 va = isp1 ? v4 : vj, vb = isp1 ? vj : v4;
+        const double4 wa = isp1 ? w4 : wj, wb = isp1 ? wj : w4;
+        const double4 h = late.h();
+        FricOut o;
+        law_friction(keff, kseff, G.mu_s, G.mu_d, G.dt, x1, pa.w, xyz(va), xyz(wa), x2, pb.w, xyz(vb),
+                     xyz(wb), mk(h.x, h.y, h.z), (((int)h.w) & 1) != 0, o);
+        if constexpr (STRESS) {  // CRotFrictionInteraction::calcSimpleForces: both forces at the contact
+          const V pos = x2 + (pb.w / eq_dist) * D;
+          const V xs = isp1 ? x1 : x2;
+          stress_add(stress, isp1 ? -1.0 * o.fn : o.fn, pos, xs);
+          stress_add(stress, isp1 ? o.Ffric : -1.0 * o.Ffric, pos, xs);
+        }
+        if (isp1) {
+          Fp += -1.0 * o.fn;
+          Mp += o.M1;
+          Fp += o.Ffric;
+          hist_out[k] = make_double4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
+                                     (o.slipping ? 1.0 : 0.0) + (o.touching ? 2.0 : 0.0));
+        } else {
+          Fp += o.fn;
+          Mp += o.M2;
+          Fp += -1.0 * o.Ffric;
+        }
+      } else {
+        const double4 b0 = late.v(), b1 = late.w();
+        const Vf vj = mk((float)b0.x, (float)b0.y, (float)b0.z), wj = mk((float)b1.x, (float)b1.y, (float)b1.z);
+        Vf hF;
+        bool hs;
+        if (EVAL) {  // evaluation pass of an FP64 run: its FP64 history
+          const double4 h = late.h();
+          hF = mk((float)h.x, (float)h.y, (float)h.z);
+          hs = (((int)h.w) & 1) != 0;
+        } else {
+          const float4 h = late.h32();
+          hF = mk(h.x, h.y, h.z);
+          hs = (((int)h.w) & 1) != 0;
+        }
+        FricOutF o;
+        law_friction_f32(keff, kseff, G.mu_s, G.mu_d, (float)G.dt, D, pa.w, pb.w, isp1 ? vself : vj,
+                         isp1 ? wself : wj, isp1 ? vj : vself, isp1 ? wj : wself, hF, hs, o);
+        if (isp1) {
+          Fk.add(-o.fn);
+          Fk.add(o.Ffric);
+          Mk.add(o.M1);
+          if (EVAL) Gs += (double)norm(o.fn) + (double)norm(o.Ffric);
+          if (!EVAL)
+            hist32_out[k] = make_float4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
+                                        (o.slipping ? 1.f : 0.f) + (o.touching ? 2.f : 0.f));
+        } else {
+          Fk.add(o.fn);
+          Fk.add(-o.Ffric);
+          Mk.add(o.M2);
+          if (EVAL) Gs += (double)norm(o.fn) + (double)norm(o.Ffric);
+        }
+      }
+    }
+  }
+}
+
 // Sum of the pair-group and bond contributions on particle i (all TPP lanes of
 // the particle call this; on return every lane holds the combined sums).  The
 // order is fixed: each lane adds its entries in adjacency order, then a
@@ -147,9 +311,7 @@ __device__ __forceinline__ void pair_sums(const StepArgs& a, const ParticleBuf& 
   Fp = mk(0.0, 0.0, 0.0);
   Mp = mk(0.0, 0.0, 0.0);
   double Gs = 0.0;  // evaluation pass: sum of the contributions' magnitudes (the particle's force scale)
-  // 3. dynamic pair groups (PIS_NE / PIS_ED::calcForces).  Contact is tested first from the
-  //    positions alone; the partner's velocity / spin and the pair's history are gathered only
-  //    for touching pairs (a non-touching RotFriction pair just resets its history).  Each lane
+  // 3. dynamic pair groups (PIS_NE / PIS_ED::calcForces), pair_entry for each entry.  Each lane
   //    takes one adjacency entry per pass (kBatch = 1); the gathers in flight come from the TPP
   //    lanes of a particle and the warps resident on the SM, not from batching within a thread.
   //    kBatch > 1 would fetch that many entries and partner positions per lane before use.
@@ -203,145 +365,8 @@ __device__ __forceinline__ void pair_sums(const StepArgs& a, const ParticleBuf& 
             }
             continue;
           }
-          const double4 pj = pjs[b];
-          // canonical orientation: p1 = lower id
-          const double4 pa = isp1 ? p4 : pj, pb = isp1 ? pj : p4;
-          const V x1 = xyz(pa), x2 = image_of(a.g, x1, xyz(pb));
-          const V D = x1 - x2;
-          const double eq_dist = pa.w + pb.w;
-          const bool touching = dot(D, D) < (eq_dist * eq_dist);  // the laws' contact test
-          if (G.kind == 0) {
-            if constexpr ((FEAT & F_ELASTIC) != 0) {
-              if (!touching) continue;
-              if constexpr (!FP32) {
-                V f;
-                if (law_elastic(elastic_k(G.k, G.scaling, pa.w, pb.w), x1, pa.w, x2, pb.w, f)) {
-                  if (isp1) Fp += -1.0 * f; else Fp += f;
-                  if constexpr (STRESS) {  // CElasticInteraction::calcForces: at x2 + r2 / (r1 + r2) D
-                    const V pos = x2 + (pb.w / eq_dist) * D;
-                    stress_add(stress, isp1 ? -1.0 * f : f, pos, isp1 ? x1 : x2);
-                  }
-                }
-              } else {
-                Vf f;
-                if (law_elastic_f32(elastic_k(G.k, G.scaling, pa.w, pb.w), D, pa.w, pb.w, f)) {
-                  Fk.add(isp1 ? -f : f);
-                  if (EVAL) Gs += (double)norm(f);
-                }
-              }
-            }
-          } else if (G.kind >= 2) {
-            // NRotFriction (CFrictionInteraction::calcForces) or HertzMindlin
-            // (CHertzMindlinInteraction::calcForces): forces only, history of the tangential force
-            if constexpr (!FP32 && (FEAT & F_NFRIC) != 0) {
-              if (!touching) {
-                if (isp1 && !EVAL) G.hist_out[k] = make_double4(0.0, 0.0, 0.0, 0.0);
-                continue;
-              }
-              const double4 vj = ldg4(in.vm + j);
-              const double4 va = isp1 ? v4 : vj, vb = isp1 ? vj : v4;
-              const double4 h = ldg4(G.hist_in + k);
-              FricOut o;
-              if (G.kind == 2) {
-                double keff, kseff;
-                nfriction_k(G.k, G.ks, G.scaling, pa.w, pb.w, keff, kseff);
-                law_nfriction(keff, kseff, G.mu_s, G.dt, x1, pa.w, xyz(va), x2, pb.w, xyz(vb), mk(h.x, h.y, h.z), o);
-              } else if (G.kind == 3) {  // E in k, nu in ks; the normal force on p1 is +fn: negated for the common form
-                law_hertz_mindlin(G.k, G.ks, G.mu_s, G.dt, x1, pa.w, xyz(va), x2, pb.w, xyz(vb), mk(h.x, h.y, h.z), o);
-                o.fn = -1.0 * o.fn;
-              } else {  // HertzMindlinVisco: E, nu, mu, restitution in k, ks, mu_s, mu_d; masses in the w's
-                law_hertz_mindlin_visco(G.k, G.ks, G.mu_s, G.mu_d, G.dt, x1, pa.w, va.w, xyz(va), x2, pb.w, vb.w, xyz(vb),
-                                        o);
-                o.fn = -1.0 * o.fn;
-              }
-              if constexpr (STRESS) {
-                const V pos = x2 + (pb.w / eq_dist) * D;
-                const V xs = isp1 ? x1 : x2;
-                stress_add(stress, isp1 ? -1.0 * o.fn : o.fn, pos, xs);
-                stress_add(stress, isp1 ? o.Ffric : -1.0 * o.Ffric, pos, xs);
-              }
-              if (isp1) {  // p1: -force, then +Ffric; p2: +force, then -Ffric
-                Fp += -1.0 * o.fn;
-                Fp += o.Ffric;
-                if (!EVAL)
-                  G.hist_out[k] = make_double4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
-                                               (o.slipping ? 1.0 : 0.0) + (o.touching ? 2.0 : 0.0));
-              } else {
-                Fp += o.fn;
-                Fp += -1.0 * o.Ffric;
-              }
-              if (EVAL) Gs += norm(o.fn) + norm(o.Ffric);
-            }
-          } else {
-            if constexpr (ROT && (FEAT & F_FRIC) != 0) {
-              if (!touching) {  // CRotFrictionInteraction::calcSimpleForces, no-contact branch
-                if (isp1 && !EVAL) {
-                  if (FP32) G.hist32_out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                  else G.hist_out[k] = make_double4(0.0, 0.0, 0.0, 0.0);
-                }
-                continue;
-              }
-              double keff, kseff;
-              friction_k(G.k, G.ks, G.scaling, G.meanR, pa.w, pb.w, keff, kseff);
-              if constexpr (!FP32) {
-                const double4 vj = ldg4(in.vm + j), wj = ldg4(in.wi + j);
-                const double4 va = isp1 ? v4 : vj, vb = isp1 ? vj : v4;
-                const double4 wa = isp1 ? w4 : wj, wb = isp1 ? wj : w4;
-                const double4 h = ldg4(G.hist_in + k);
-                FricOut o;
-                law_friction(keff, kseff, G.mu_s, G.mu_d, G.dt, x1, pa.w, xyz(va), xyz(wa), x2, pb.w, xyz(vb),
-                             xyz(wb), mk(h.x, h.y, h.z), (((int)h.w) & 1) != 0, o);
-                if constexpr (STRESS) {  // CRotFrictionInteraction::calcSimpleForces: both forces at the contact
-                  const V pos = x2 + (pb.w / eq_dist) * D;
-                  const V xs = isp1 ? x1 : x2;
-                  stress_add(stress, isp1 ? -1.0 * o.fn : o.fn, pos, xs);
-                  stress_add(stress, isp1 ? o.Ffric : -1.0 * o.Ffric, pos, xs);
-                }
-                if (isp1) {
-                  Fp += -1.0 * o.fn;
-                  Mp += o.M1;
-                  Fp += o.Ffric;
-                  G.hist_out[k] = make_double4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
-                                               (o.slipping ? 1.0 : 0.0) + (o.touching ? 2.0 : 0.0));
-                } else {
-                  Fp += o.fn;
-                  Mp += o.M2;
-                  Fp += -1.0 * o.Ffric;
-                }
-              } else {
-                const double4 b0 = ldg4(in.vm + j), b1 = ldg4(in.wi + j);
-                const Vf vj = mk((float)b0.x, (float)b0.y, (float)b0.z), wj = mk((float)b1.x, (float)b1.y, (float)b1.z);
-                Vf hF;
-                bool hs;
-                if (EVAL) {  // evaluation pass of an FP64 run: its FP64 history
-                  const double4 h = ldg4(G.hist_in + k);
-                  hF = mk((float)h.x, (float)h.y, (float)h.z);
-                  hs = (((int)h.w) & 1) != 0;
-                } else {
-                  const float4 h = __ldg(G.hist32_in + k);
-                  hF = mk(h.x, h.y, h.z);
-                  hs = (((int)h.w) & 1) != 0;
-                }
-                FricOutF o;
-                law_friction_f32(keff, kseff, G.mu_s, G.mu_d, (float)G.dt, D, pa.w, pb.w, isp1 ? vself : vj,
-                                 isp1 ? wself : wj, isp1 ? vj : vself, isp1 ? wj : wself, hF, hs, o);
-                if (isp1) {
-                  Fk.add(-o.fn);
-                  Fk.add(o.Ffric);
-                  Mk.add(o.M1);
-                  if (EVAL) Gs += (double)norm(o.fn) + (double)norm(o.Ffric);
-                  if (!EVAL)
-                    G.hist32_out[k] = make_float4(o.Ffric.x, o.Ffric.y, o.Ffric.z,
-                                                  (o.slipping ? 1.f : 0.f) + (o.touching ? 2.f : 0.f));
-                } else {
-                  Fk.add(o.fn);
-                  Fk.add(-o.Ffric);
-                  Mk.add(o.M2);
-                  if (EVAL) Gs += (double)norm(o.fn) + (double)norm(o.Ffric);
-                }
-              }
-            }
-          }
+          pair_entry<ROT, FEAT, FP32, EVAL>(a.g, G, k, isp1, p4, pjs[b], v4, w4, vself, wself, G.hist_out, G.hist32_out,
+                                            PairGather{in, G, j, k}, Fp, Mp, Fk, Mk, Gs, stress);
         }
       }
     }
@@ -359,7 +384,8 @@ __device__ __forceinline__ void pair_sums(const StepArgs& a, const ParticleBuf& 
           // a bond removed by an earlier update carries zero records (bond_pass_one writes them)
           if constexpr (FP32 && !EVAL) {
             const float4* rf = B.bf32 + 4 * (size_t)k + (en.y < 0 ? 0 : 2);
-            const float4 a0 = __ldg(rf), a1 = __ldg(rf + 1);
+            float4 a0, a1;
+            ldg8(rf, a0, a1);
             Fp += mk((double)a0.x, (double)a0.y, (double)a0.z);
             if (ROT) Mp += mk((double)a0.w, (double)a1.x, (double)a1.y);
             continue;
@@ -690,7 +716,8 @@ __device__ __forceinline__ void pair_sums_warp(const StepArgs& a, const Particle
           const int k = en.y & 0x7fffffff;
           if constexpr (FP32 && !EVAL) {
             const float4* rf = B.bf32 + 4 * (size_t)k + (en.y < 0 ? 0 : 2);
-            const float4 a0 = __ldg(rf), a1 = __ldg(rf + 1);
+            float4 a0, a1;
+            ldg8(rf, a0, a1);
             Fp += mk((double)a0.x, (double)a0.y, (double)a0.z);
             if (ROT) Mp += mk((double)a0.w, (double)a1.x, (double)a1.y);
             continue;
@@ -714,6 +741,98 @@ __device__ __forceinline__ void pair_sums_warp(const StepArgs& a, const Particle
     Mp = Mk.value() + Mp;
   }
   if (EVAL && gross) *gross = Gs;
+}
+
+// 1. elastic walls on one particle, in group-name order (TSubLattice::calcForces,
+//    SubLattice.hpp:2116-2120): adds the wall forces to F.  Every thread of the block calls this
+//    (`on`: it carries a particle); the walls' reactions are reduced in a fixed order: warp
+//    shuffle, then warps, then blocks.
+template <bool EVAL>
+__device__ __forceinline__ void wall_forces(int nwall, const WallDev* walls, bool on, unsigned pf, const V& xi, double r,
+                                            int wlane, int warp, double (*s_red)[kMaxWalls][3], V& F) {
+  for (int w = 0; w < nwall; ++w) {
+    V c = mk(0.0, 0.0, 0.0);
+    if (on && (pf & (1u << (PF_WALL_SHIFT + w)))) {
+      const WallDev W = walls[w];
+      V f;
+      if (law_wall(W.k, mk(W.ox, W.oy, W.oz), mk(W.nx, W.ny, W.nz), xi, r, f)) {
+        F += f;
+        if (pf & (1u << (PF_INNER_SHIFT + w))) c = f;  // CWall::addForce(-F): m_force -= -F
+      }
+    }
+    if (!EVAL) {
+      double cx = c.x, cy = c.y, cz = c.z;
+      if (__any_sync(0xffffffffu, cx != 0.0 || cy != 0.0 || cz != 0.0)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          cx += __shfl_down_sync(0xffffffffu, cx, o);
+          cy += __shfl_down_sync(0xffffffffu, cy, o);
+          cz += __shfl_down_sync(0xffffffffu, cz, o);
+        }
+      }
+      if (wlane == 0) { s_red[warp][w][0] += cx; s_red[warp][w][1] += cy; s_red[warp][w][2] += cz; }
+    }
+  }
+}
+
+// 5. damping, last (SubLattice.hpp:2140-2145), in the damping map's name order: on the force
+//    "Damping" and a LocalDamping group (by its own name); on the moment "RotDamping" then
+//    "RotLocalDamping".  iv = 1/m, 1/I.
+template <bool ROT>
+__device__ __forceinline__ void damp(const StepArgs& a, const double4& v4, const double4& w4, const double2& iv, V& F,
+                                     V& M, int& it_lin, int& it_rot) {
+  it_lin = it_rot = 0;
+  if (a.damp_loc && a.loc_before_lin) F += local_damping_force(xyz(v4), F, a.visc_loc);
+  if (a.damp_lin) F += damping_force(xyz(v4), F, iv.x, v4.w, a.visc_lin, a.dt_lin, a.iter_lin, &it_lin);
+  if (a.damp_loc && !a.loc_before_lin) F += local_damping_force(xyz(v4), F, a.visc_loc);
+  if (ROT && a.damp_rot) M += damping_force(xyz(w4), M, iv.y, w4.w, a.visc_rot, a.dt_rot, a.iter_rot, &it_rot);
+  if (ROT && a.damp_rotloc) M += local_damping_force(xyz(w4), M, a.visc_rotloc);
+}
+
+// 6. integration (CRotParticle::integrate + rescale, RotParticle.cpp:277-321; Particle.cpp:257-274).
+//    turn_quat: the orientation under the new spin w.
+__device__ __forceinline__ void turn_quat(unsigned pf, double dt, const V& w, double4& q4) {
+  Qd q{q4.x, mk(q4.y, q4.z, q4.w)};
+  if (pf & PF_ROT) {
+    const Qd dq = qmul(Qd{0.0, w}, q);
+    const double c = dt / 2.0;
+    q.s += c * dq.s;
+    q.v += c * dq.v;
+  }
+  const double module = sqrt(q.s * q.s + q.v.x * q.v.x + q.v.y * q.v.y + q.v.z * q.v.z);
+  if (module != 0.0) {
+    const double inverse = 1.0 / module;
+    q.s = inverse * q.s;
+    q.v = inverse * q.v;
+  }
+  q4 = make_double4(q.s, q.v.x, q.v.y, q.v.z);
+}
+__device__ __forceinline__ void integrate_spin(unsigned pf, double dt, double inv_i, const V& M, V& w) {
+  if (pf & PF_ROT) w += (dt * inv_i) * M;
+  else w = mk(0.0, 0.0, 0.0);
+}
+__device__ __forceinline__ void integrate_lin(unsigned pf, double dt, double inv_m, const V& F, V& v, V& x) {
+  if (pf & PF_DYN) {
+    v += F * inv_m * dt;
+    x += v * dt;
+  }
+}
+
+// 7. displacement check for the next step (TSubLattice::checkNeighbors): |x - oldpos| >
+//    verletDist/2, evaluated exactly whenever the running bound of it (this step's
+//    displacement added to the bound, in FP32 rounded up) does not already rule it out.
+//    The difference of a position before and after one step is exact (the two are close), so
+//    rounding the norm up at each FP32 operation keeps it a bound.  b: the bound, updated;
+//    returns whether the next step must search.
+__device__ __forceinline__ bool displaced(const StepArgs& a, int i, const V& xi, const V& x, float& b) {
+  const float dx = __double2float_ru(fabs(x.x - xi.x)), dy = __double2float_ru(fabs(x.y - xi.y)),
+              dz = __double2float_ru(fabs(x.z - xi.z));
+  const float len = __fsqrt_ru(__fmaf_ru(dx, dx, __fmaf_ru(dy, dy, __fmul_ru(dz, dz))));
+  b = __fadd_ru(b, __fmul_ru(len, 1.0000005f));
+  if ((double)b * (double)b < a.half_alpha_sq * 0.999999) return false;
+  const double4 op = ldg4(a.P.oldpos + i);
+  const V dd = mk(x.x - op.x, x.y - op.y, x.z - op.z);
+  return dot(dd, dd) > a.half_alpha_sq;
 }
 
 // Walls, body force, the pair sums, damping and the integration of particle i
@@ -753,31 +872,7 @@ __device__ __forceinline__ void finish_particle(const StepArgs& a, long long ste
   }
   if (a.pf_log && lane == 0 && i < a.P.n) a.pf_log[i] = pf;
 
-  // 1. elastic walls, in group-name order (TSubLattice::calcForces, SubLattice.hpp:2116-2120).
-  //    The walls' reactions are reduced in a fixed order: warp shuffle, then warps, then blocks.
-  for (int w = 0; w < a.nwall; ++w) {
-    V c = mk(0.0, 0.0, 0.0);
-    if (alive && lane == 0 && (pf & (1u << (PF_WALL_SHIFT + w)))) {
-      const WallDev W = a.walls[w];
-      V f;
-      if (law_wall(W.k, mk(W.ox, W.oy, W.oz), mk(W.nx, W.ny, W.nz), xi, p4.w, f)) {
-        F += f;
-        if (pf & (1u << (PF_INNER_SHIFT + w))) c = f;  // CWall::addForce(-F): m_force -= -F
-      }
-    }
-    if (!EVAL) {
-      double cx = c.x, cy = c.y, cz = c.z;
-      if (__any_sync(0xffffffffu, cx != 0.0 || cy != 0.0 || cz != 0.0)) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          cx += __shfl_down_sync(0xffffffffu, cx, o);
-          cy += __shfl_down_sync(0xffffffffu, cy, o);
-          cz += __shfl_down_sync(0xffffffffu, cz, o);
-        }
-      }
-      if (wlane == 0) { s_red[warp][w][0] += cx; s_red[warp][w][1] += cy; s_red[warp][w][2] += cz; }
-    }
-  }
+  wall_forces<EVAL>(a.nwall, a.walls, alive && lane == 0, pf, xi, p4.w, wlane, warp, s_red, F);
 
   // 2. body forces (BodyForceGroup::calcForces, BodyForceGroup.hpp:54-65): F += g * m
   if (alive && lane == 0)
@@ -792,15 +887,8 @@ __device__ __forceinline__ void finish_particle(const StepArgs& a, long long ste
       a.f_int[i] = d4(F, 0.0);
       a.m_int[i] = d4(M, 0.0);
     }
-    // 5. damping, last (SubLattice.hpp:2140-2145), in the damping map's name order: on the force
-    //    "Damping" and a LocalDamping group (by its own name); on the moment "RotDamping" then
-    //    "RotLocalDamping"
-    int it_lin = 0, it_rot = 0;
-    if (a.damp_loc && a.loc_before_lin) F += local_damping_force(xyz(v4), F, a.visc_loc);
-    if (a.damp_lin) F += damping_force(xyz(v4), F, iv.x, v4.w, a.visc_lin, a.dt_lin, a.iter_lin, &it_lin);
-    if (a.damp_loc && !a.loc_before_lin) F += local_damping_force(xyz(v4), F, a.visc_loc);
-    if (ROT && a.damp_rot) M += damping_force(xyz(w4), M, iv.y, w4.w, a.visc_rot, a.dt_rot, a.iter_rot, &it_rot);
-    if (ROT && a.damp_rotloc) M += local_damping_force(xyz(w4), M, a.visc_rotloc);
+    int it_lin, it_rot;
+    damp<ROT>(a, v4, w4, iv, F, M, it_lin, it_rot);
     if (a.damp_iters) {
       a.damp_iters[2 * i] = (unsigned char)(it_lin > 255 ? 255 : it_lin);
       a.damp_iters[2 * i + 1] = (unsigned char)(it_rot > 255 ? 255 : it_rot);
@@ -809,37 +897,19 @@ __device__ __forceinline__ void finish_particle(const StepArgs& a, long long ste
       a.P.force_eval[i] = d4(F, 0.0);
       if (ROT) a.P.moment_eval[i] = d4(M, 0.0);
     } else {
-      // 6. integration (CRotParticle::integrate + rescale, RotParticle.cpp:277-321; Particle.cpp:257-274)
       const double dt = a.dt;
       V v = xyz(v4), x = xi;
       V w = xyz(w4);
       if (ROT) {
         if (!q_loaded) q4 = ldg4(in.qq + i);
-        Qd q{q4.x, mk(q4.y, q4.z, q4.w)};
-        if (pf & PF_ROT) {
-          w += (dt * iv.y) * M;
-          const Qd dq = qmul(Qd{0.0, w}, q);
-          const double c = dt / 2.0;
-          q.s += c * dq.s;
-          q.v += c * dq.v;
-        } else {
-          w = mk(0.0, 0.0, 0.0);
-        }
-        const double module = sqrt(q.s * q.s + q.v.x * q.v.x + q.v.y * q.v.y + q.v.z * q.v.z);
-        if (module != 0.0) {
-          const double inverse = 1.0 / module;
-          q.s = inverse * q.s;
-          q.v = inverse * q.v;
-        }
-        out.wi[i] = d4(w, w4.w);
-        out.qq[i] = make_double4(q.s, q.v.x, q.v.y, q.v.z);
+        integrate_spin(pf, dt, iv.y, M, w);
+        turn_quat(pf, dt, w, q4);
+        st4(out.wi + i, d4(w, w4.w));
+        st4(out.qq + i, q4);
       }
-      if (pf & PF_DYN) {
-        v += F * iv.x * dt;
-        x += v * dt;
-      }
-      out.pr[i] = d4(x, p4.w);
-      out.vm[i] = d4(v, v4.w);
+      integrate_lin(pf, dt, iv.x, F, v, x);
+      st4(out.pr + i, d4(x, p4.w));
+      st4(out.vm + i, d4(v, v4.w));
       if (FP32 && !a.skip_vw) {
         out.vw[2 * i] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)w.x);
         out.vw[2 * i + 1] = make_float4((float)w.y, (float)w.z, 0.f, 0.f);
@@ -848,19 +918,9 @@ __device__ __forceinline__ void finish_particle(const StepArgs& a, long long ste
         a.P.force[i] = d4(F, 0.0);
         if (ROT) a.P.moment[i] = d4(M, 0.0);
       }
-      // 7. displacement check for the next step (TSubLattice::checkNeighbors): |x - oldpos| >
-      //    verletDist/2, evaluated exactly whenever the running bound of it (this step's
-      //    displacement added to the bound, in FP32 rounded up) does not already rule it out.
-      //    The difference of a position before and after one step is exact (the two are close),
-      //    so the bound only has to cover the norm's rounding.
-      const V sd = mk(x.x - xi.x, x.y - xi.y, x.z - xi.z);
-      const float b = __fadd_ru(a.P.dbound[i], __fmul_ru(__double2float_ru(sqrt(dot(sd, sd))), 1.0000005f));
+      float b = a.P.dbound[i];
+      if (displaced(a, i, xi, x, b)) atomicOr(a.ctrl, CTRL_REBUILD);
       a.P.dbound[i] = b;
-      if ((double)b * (double)b >= a.half_alpha_sq * 0.999999) {
-        const double4 op = ldg4(a.P.oldpos + i);
-        const V dd = mk(x.x - op.x, x.y - op.y, x.z - op.z);
-        if (dot(dd, dd) > a.half_alpha_sq) atomicOr(a.ctrl, CTRL_REBUILD);
-      }
     }
   }
 }
@@ -889,6 +949,7 @@ __device__ __forceinline__ void wall_totals(const StepArgs& a, long long step, i
 // This block's wall partials (fixed order over warps) into slot `part`, then the
 // last-arriving block of the `nparts` is detected on `counter`.  Returns true in that block.
 // All threads of the block call this.
+template <int WARPS = kStepWarps>
 __device__ __forceinline__ bool block_partials(const StepArgs& a, int part, int nparts, unsigned* counter,
                                                double (*s_red)[kMaxWalls][3], bool* s_last) {
   const int nw3 = a.nwall * 3;
@@ -896,7 +957,7 @@ __device__ __forceinline__ bool block_partials(const StepArgs& a, int part, int 
   if (threadIdx.x < nw3) {
     const int w = threadIdx.x / 3, c = threadIdx.x % 3;
     double acc = 0.0;
-    for (int k = 0; k < kStepWarps; ++k) acc += s_red[k][w][c];
+    for (int k = 0; k < WARPS; ++k) acc += s_red[k][w][c];
     a.wall_partial[((size_t)part * kMaxWalls + w) * 3 + c] = acc;
   }
   __syncthreads();
@@ -957,9 +1018,9 @@ __device__ __forceinline__ void store_bond(const BondDev& B, int k, const V& f, 
     r[3] = make_float4((float)m2.y, (float)m2.z, 0.f, 0.f);
   } else {
     double4* r = B.bf + 3 * (size_t)k;
-    r[0] = d4(f, 0.0);
-    r[1] = d4(m1, 0.0);
-    r[2] = d4(m2, 0.0);
+    st4(r, d4(f, 0.0));
+    st4(r + 1, d4(m1, 0.0));
+    st4(r + 2, d4(m2, 0.0));
   }
 }
 

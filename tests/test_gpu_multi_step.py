@@ -1,0 +1,92 @@
+"""The multi-step kernel (bond-free specimens) against single-step launches of the same timesteps.
+
+Both form every particle's sums in the same order, so the FP64 states are equal bit for bit,
+whatever the block's share of particles, its pruned lists, their refreshes and the neighbour
+searches in between.  Wall reactions are summed over blocks of different sizes: each is compared
+within n * 2^-52 of the sum's scale.  The FP32-force form differs by FMA contraction only: its
+rounding (2^-24 per operation, about 40 operations and 20 contributions a force) stays below 1e-5
+of the largest force.
+"""
+import numpy as np
+import pytest
+
+import scenarios as S
+from conftest import gpu_available
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu(dem_lib):
+    if not gpu_available():
+        pytest.skip("no GPU")
+    from esys.lsm import _capi
+
+    return lambda *a: _capi.DemSim(*a)
+
+
+def _pair(gpu, build, kw, steps, prec=64):
+    out = []
+    for single in (False, True):
+        s = build(gpu, **kw)
+        if prec != 64:
+            s.set_option("precision", prec)
+        if single:
+            s.set_option("split", 1)  # two single-step kernels a step (one where the law has no split form)
+        for k in steps:
+            s.step(k)
+        out.append(s)
+    return out
+
+
+def _equal(a, b, groups, walls):
+    pa, pb = a.particles(), b.particles()
+    for k in pa:
+        assert np.array_equal(pa[k], pb[k]), (k, np.abs(pa[k] - pb[k]).max())
+    for g in groups:
+        for x, y in zip(a.pairs(g), b.pairs(g)):
+            assert np.array_equal(x, y), g
+    assert a.counters()["rebuilds"] == b.counters()["rebuilds"]
+    n = len(pa["id"])
+    for w in walls:
+        (xa, fa), (xb, fb) = a.wall(w), b.wall(w)
+        assert np.array_equal(xa, xb)
+        assert np.abs(fa - fb).max() <= n * 2.0 ** -52 * max(np.abs(fb).max(), 1e-300)
+
+
+FR = (["friction"], ["floor", "roof"])
+CASES = [
+    # one particle; fewer particles than a block's groups; a ragged count over many blocks
+    ("one", S.friction_pack, dict(nx=1, ny=1, nz=1), (5,), FR),
+    ("seven", S.friction_pack, dict(nx=7, ny=1, nz=1), (1, 2, 30), FR),
+    ("ragged", S.friction_pack, dict(nx=13, ny=11, nz=12), (60,), FR),
+    ("periodic", S.friction_pack, dict(nx=9, ny=6, nz=7, periodic=True, vscale=30.0), (90, 1, 40), FR),
+    # fast: the lists are pruned again and neighbour searches stop the launch every few steps
+    ("fast", S.friction_pack, dict(nx=10, ny=9, nz=8, vscale=250.0), (64,), FR),
+    ("elastic", S.gravity_box, dict(n_side=9), (120,), (["elastic"], ["xlo", "zlo", "zhi"])),
+    ("nrot_friction", S.nrot_friction_pack, dict(n_side=7, vscale=20.0), (80,), (["friction"], [])),
+    ("rot_nrot_friction", S.nrot_friction_pack, dict(rot=True, n_side=5), (50,), (["friction"], [])),
+    ("hertz", S.hertz_mindlin_pack, dict(n_side=6, vscale=20.0), (80,), ([], [])),
+    # two halves of a block no longer hold the particles; records read back from L2: results in
+    # several parts (dense), all at once (loose), and entries beyond a block's room (densest)
+    ("block_256_up", S.friction_pack, dict(nx=36, ny=34, nz=35, squeeze=1.1), (30,), FR),
+    ("parts", S.friction_pack, dict(nx=44, ny=40, nz=40), (12,), FR),
+    ("loose", S.friction_pack, dict(nx=70, ny=50, nz=50, squeeze=1.14), (12,), FR),
+    ("beyond", S.friction_pack, dict(nx=64, ny=44, nz=44, squeeze=0.8), (8,), FR),
+]
+
+
+@pytest.mark.parametrize("name,build,kw,steps,what", CASES, ids=[c[0] for c in CASES])
+def test_equals_single_steps(gpu, name, build, kw, steps, what):
+    a, b = _pair(gpu, build, kw, steps)
+    _equal(a, b, *what)
+
+
+@pytest.mark.parametrize("kw,steps", [(dict(nx=13, ny=11, nz=12), 40), (dict(nx=70, ny=50, nz=50, squeeze=1.14), 12)])
+def test_fp32_form_equals_single_steps(gpu, kw, steps):
+    a, b = _pair(gpu, S.friction_pack, kw, (steps,), prec=32)
+    pa, pb = a.particles(), b.particles()
+    for k in ("pos", "vel", "angvel", "force", "moment"):
+        assert np.abs(pa[k] - pb[k]).max() <= 1e-5 * np.abs(pb[k]).max(), k
+    for x, y in zip(a.pairs("friction")[:2], b.pairs("friction")[:2]):
+        assert np.array_equal(x, y)
