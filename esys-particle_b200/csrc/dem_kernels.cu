@@ -11,6 +11,7 @@
 //  k_bin ... k_adj_*   the neighbour search / interaction update
 //                      (ntable/src/ntable.hpp:262-664, pis/pi_storage_ne.hpp:49-102,
 //                      pis/pi_storage_ed.hpp:84-161).
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 
@@ -462,6 +463,35 @@ __global__ void k_pack_particles(Particles P, int cur, int rot, const int* rows,
   }
 }
 
+// k_pack_particles' rows written to host-mapped memory: consecutive threads write consecutive
+// doubles, so the bus carries whole lines.  blockIdx.y is the field (6: ids).  Bound by the bus (a
+// few us for a small specimen, about 50 GB/s for a large one).
+__global__ void k_rows_direct(Particles P, int cur, int rot, const ParticleRows to) {
+  const int f = blockIdx.y;
+  const ParticleBuf b = P.buf[cur];
+  if (f == 6) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; to.id && i < P.n; i += gridDim.x * blockDim.x) to.id[i] = P.id[i];
+    return;
+  }
+  double* const dst = to.field[f];
+  if (!dst) return;
+  const double4* const src[6] = {b.pr, b.vm, b.wi, b.qq, P.force, P.moment};
+  const int w = f == 3 ? 4 : 3;
+  const bool spin = f == 2 || f == 3 || f == 5;  // a non-rotational particle: zero, and the identity quaternion
+  const int total = P.n * w;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+    const int i = e / w, c = e % w;
+    dst[e] = spin && !rot ? (f == 3 && c == 0 ? 1.0 : 0.0) : reinterpret_cast<const double*>(src[f] + i)[c];
+  }
+}
+
+__global__ void k_wall_state(const WallDev* walls, const double* wall_force, int nw, double* to) {
+  const int w = threadIdx.x / 6, c = threadIdx.x % 6;
+  if (w >= nw) return;
+  const WallDev& W = walls[w];
+  to[threadIdx.x] = c == 0 ? W.ox : c == 1 ? W.oy : c == 2 ? W.oz : wall_force[3 * w + c - 3];
+}
+
 // Displacement check after a host-side move (TSubLattice::checkNeighbors).
 __global__ void k_check_disp(Particles P, int cur, double half_alpha_sq, int* ctrl) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -779,6 +809,12 @@ void launch_pack_particles(const Particles& P, int cur, int rot, const int* rows
                            double* angvel, double* quat, double* force, double* moment, cudaStream_t s) {
   if (P.n)
     k_pack_particles<<<nblk(P.n, 256), 256, 0, s>>>(P, cur, rot, rows, id, pos, vel, angvel, quat, force, moment);
+}
+void launch_rows_direct(const Particles& P, int cur, int rot, const ParticleRows& to, cudaStream_t s) {
+  if (P.n) k_rows_direct<<<dim3(std::min(nblk(4LL * P.n, 256), 148), 7), 256, 0, s>>>(P, cur, rot, to);
+}
+void launch_wall_state(const WallDev* walls, const double* wall_force, int nw, double* to, cudaStream_t s) {
+  k_wall_state<<<1, 64, 0, s>>>(walls, wall_force, nw, to);
 }
 void launch_check_disp(const Particles& P, int cur, double half_alpha_sq, int* ctrl, cudaStream_t s) {
   if (P.n) k_check_disp<<<nblk(P.n, 256), 256, 0, s>>>(P, cur, half_alpha_sq, ctrl);

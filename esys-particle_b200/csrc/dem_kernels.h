@@ -42,6 +42,15 @@ void launch_alive_flags(const Particles& P, int* flags, cudaStream_t s);
 void launch_set_alive(const Particles& P, int cnt, const int* slots, cudaStream_t s);
 void launch_pack_particles(const Particles& P, int cur, int rot, const int* rows, int* id, double* pos, double* vel,
                            double* angvel, double* quat, double* force, double* moment, cudaStream_t s);
+// Rows of every slot (all alive) straight into host-mapped arrays, each null or device-addressable:
+// position, velocity, spin, quaternion (4 a row), force, moment, and ids.
+struct ParticleRows {
+  double* field[6];
+  int* id;
+};
+void launch_rows_direct(const Particles& P, int cur, int rot, const ParticleRows& to, cudaStream_t s);
+// The wall groups' origins and last reactions, 6 doubles each, to `to` (host-mapped).
+void launch_wall_state(const WallDev* walls, const double* wall_force, int nw, double* to, cudaStream_t s);
 void launch_check_disp(const Particles& P, int cur, double half_alpha_sq, int* ctrl, cudaStream_t s);
 void launch_move_tagged(const Particles& P, int cur, int tag, const double* d, cudaStream_t s);
 // idx: scratch of at least P.n ints (each servo thread's candidate list)

@@ -184,6 +184,7 @@ struct DemSim {
   unsigned long long* d_run = nullptr;
   int num_sms = 0;       // of the current device; 0 until asked for
   int* h_ctrl = nullptr;  // pinned
+  double* h_walls = nullptr;  // pinned: the wall groups' origins and reactions (6 each) as a kernel writes them
   long long t = 0;
   int timestamp = 0, last_ns = -1;
   bool first = true;
@@ -204,6 +205,7 @@ struct DemSim {
   DemSim() {
     DEM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     DEM_CUDA(cudaMallocHost(&h_ctrl, 4 * sizeof(long long)));
+    DEM_CUDA(cudaMallocHost(&h_walls, 6 * kMaxWalls * sizeof(double)));
     d_block_counter.reserve(1); d_ctl.reserve(4); scalars.reserve(8);
     d_step = d_ctl.p;
     d_ctrl = reinterpret_cast<int*>(d_ctl.p + 1);
@@ -231,6 +233,7 @@ struct DemSim {
     stage.release(); stage_slot.release(); scratch_d.release(); sig.release(); d_servo_idx.release(); d_brk.release(); rows.release(); pack_id.release();
     pack.release();
     if (h_ctrl) cudaFreeHost(h_ctrl);
+    if (h_walls) cudaFreeHost(h_walls);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (own_stream) cudaStreamDestroy(s);
@@ -527,23 +530,58 @@ struct DemSim {
     if (!id) throw std::invalid_argument("revive needs particle ids");
     set_particles(cnt, id, pos, vel, angvel, quat);  // uploads the slots to stage_slot
     launch_set_alive(P, cnt, stage_slot.p, s);
+    alive_n = -1;
     pending_ctrl |= CTRL_REBUILD;
     sync();
     c_launches += 1;
     return 0;
   }
 
-  // The alive particles in slot order into the caller's host arrays (each may be null).  The
+  // The device address of page-locked host memory, or null for any other.
+  template <class T>
+  static T* mapped(T* host) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<T*>(at.devicePointer) : nullptr;
+  }
+
+  // The alive particles in slot order into the caller's host arrays (each may be null).  A specimen
+  // of up to kDirectRows rows read into page-locked arrays is written there by one kernel: the copy
+  // engine's latency for up to seven fields, one after another, was most of such a call.  Otherwise the
   // rows are packed on the device, then each wanted field is one copy into the caller's array
   // (direct DMA when the caller's memory is pinned).
+  static constexpr int kDirectRows = 1 << 16;
+  int alive_n = -1;  // alive particles; -1: to be counted (only a neighbour search or a revival changes them)
   int get_particles(int* id, double* pos, double* vel, double* angvel, double* quat, double* force, double* moment) {
     if (!n) return 0;
     rows.reserve((size_t)n + 1);
     pack_id.reserve((size_t)n + 1);
-    scan_tmp.reserve(scan_tmp_ints(n + 1));
-    launch_alive_flags(P, pack_id.p, s);  // flags, then the scan's input is free for the ids
-    launch_scan(pack_id.p, rows.p, n, scalars.p + 2, scan_tmp.p, s);
-    const int k = read_int(scalars.p + 2);
+    if (alive_n < 0) {
+      scan_tmp.reserve(scan_tmp_ints(n + 1));
+      launch_alive_flags(P, pack_id.p, s);  // flags, then the scan's input is free for the ids
+      launch_scan(pack_id.p, rows.p, n, scalars.p + 2, scan_tmp.p, s);
+      alive_n = read_int(scalars.p + 2);
+      c_launches += 2;
+    }
+    const int k = alive_n;
+    if (k == n && n <= kDirectRows) {
+      ParticleRows to{};
+      double* const want[6] = {pos, vel, angvel, quat, force, moment};
+      bool all = true;
+      for (int f = 0; f < 6 && all; ++f)
+        if (want[f]) all = (to.field[f] = mapped(want[f])) != nullptr;
+      if (id && all) all = (to.id = mapped(id)) != nullptr;
+      if (all) {
+        launch_rows_direct(P, cur, rot, to, s);
+        DEM_CUDA(cudaGetLastError());
+        sync();
+        c_launches += 1;
+        return k;
+      }
+    }
     const int* rp = k == n ? nullptr : rows.p;  // every slot alive: row = slot
     pack.reserve((size_t)19 * n + 1);
     double* d = pack.p;
@@ -564,12 +602,13 @@ struct DemSim {
     if (force) DEM_CUDA(cudaMemcpyAsync(force, dfor, k3, cudaMemcpyDeviceToHost, s));
     if (moment) DEM_CUDA(cudaMemcpyAsync(moment, dmom, k3, cudaMemcpyDeviceToHost, s));
     sync();
-    c_launches += 3;
+    c_launches += 1;
     return k;
   }
 
   // ---- neighbour search (TSubLattice::searchNeighbors, SubLattice.hpp:2395-2408) ----
   void search_neighbors() {
+    alive_n = -1;
     DEM_CUDA(cudaMemsetAsync(cell_count.p, 0, sizeof(int) * (ncell + 1), s));
     launch_bin(g, P, cur, cell_count.p, s);
     scan_tmp.reserve(scan_tmp_ints(std::max(ncell + 1, n + 2)));
@@ -717,16 +756,21 @@ struct DemSim {
     }
     sync();
   }
-  // device wall origins are authoritative once groups exist: bring them back to the host
-  void download_walls() {
+  // device wall origins are authoritative once groups exist: bring them back to the host, with the
+  // groups' last reactions (3 each) where `force` is given
+  void download_walls(double* force = nullptr) {
     if (wig.empty()) return;
-    std::vector<WallDev> w(wig.size());
-    DEM_CUDA(cudaMemcpyAsync(w.data(), d_walls.p, sizeof(WallDev) * w.size(), cudaMemcpyDeviceToHost, s));
+    const int nw = (int)wig.size();
+    launch_wall_state(d_walls.p, d_wall_force.p, nw, h_walls, s);
+    DEM_CUDA(cudaGetLastError());
     sync();
     int k = 0;
     for (auto& it : wig) {
       Wall& W = walls.at(it.second.wall);
-      W.o[0] = w[k].ox; W.o[1] = w[k].oy; W.o[2] = w[k].oz;
+      for (int c = 0; c < 3; ++c) {
+        W.o[c] = h_walls[6 * k + c];
+        if (force) force[3 * k + c] = h_walls[6 * k + 3 + c];
+      }
       ++k;
     }
   }
@@ -3028,10 +3072,8 @@ int dem_apply_force_to_wall(dem_sim* h, const char* group, const double* f) {
 int dem_get_wall(dem_sim* h, const char* name, double* pos, double* force) {
   return guard(h, [&](DemSim& s) {
     if (!s.walls.count(name)) throw std::invalid_argument("no such wall");
-    s.download_walls();
-    double wf[dem::kMaxWalls * 3];
-    DEM_CUDA(cudaMemcpyAsync(wf, s.d_wall_force.p, sizeof(wf), cudaMemcpyDeviceToHost, s.s));
-    s.sync();
+    double wf[dem::kMaxWalls * 3] = {0};
+    s.download_walls(wf);
     double F[3] = {0, 0, 0};
     int k = 0;
     for (auto& it : s.wig) {
