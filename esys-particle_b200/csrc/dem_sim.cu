@@ -136,6 +136,7 @@ struct DemSim {
   int tpp = 0;           // 0 = choose from the mean adjacency length
   int chunk = 0;         // steps launched per host round trip ("chunk"); 0 = kChunk, or kRunChunk in one multi-step launch
   static constexpr int kChunk = 64, kRunChunk = 1024;
+  static constexpr double kRunDense = 4.5;  // mean entries from which an FP64 frictional packing takes single steps
   static constexpr int kRunMin = 4;        // multi-step kernel without resident records: fewer steps go out singly
   static constexpr int kRunEntries = 256;  // list entries per block that a small specimen's block count aims at
   // The multi-step kernel stays off until this neighbour search (counted by timestamp) after a launch
@@ -1028,6 +1029,11 @@ struct DemSim {
     }
     // else the records stay in L2, and what is left is shared 60:40 between entries and results
     ra.one = 0;
+    // A dense frictional packing in FP64 does not gain: nearly every listed pair touches, so pruning leaves
+    // the lists as long, and the law, evaluated for both owners, sets the pace of either kernel (40 steps of
+    // 64,000 particles with 5.8 entries each: 1333 us here, 1126 singly; 100 steps of 125,000 with 3.4:
+    // 1718 here, 2893 singly; in the FP32 form the former take 1018 and 1155).
+    if (!fp32 && fric && mean >= kRunDense) return false;
     const size_t fixed = run_layout(rot, fric, moment, fp32, false, ra.ppb, 0, 0).bytes + 128;
     if (ra.ppb > 65535 || fixed > kSmem / 2) return false;
     const size_t left = kSmem - fixed, res = (size_t)(fp32 ? 4 : 8) * (moment ? 9 : (fric ? 6 : 3));
