@@ -89,7 +89,8 @@ struct DynGroup {
   DBuf<unsigned long long> keys, keys_spare, cand;
   DBuf<double4> hist[2], hist_spare;  // hist[c]: read by the step whose particle input buffer is c
   DBuf<float4> hist32[2], hist32_spare;  // the same records in the FP32-force form
-  DBuf<int> adj_start, adj_count, adj_cursor, p1_start;
+  DBuf<int> adj_start, adj_count, adj_cursor, p1_start, p1_spare;
+  int p1_n = -1;  // the particles that p1_start holds the list's ranges of; -1: not this list's
   DBuf<int2> adj;
   DBuf<int> xbond;  // device bond hand-off: excluding bond of each pair
   DBuf<int2> adj_free;  // and each particle's free entries
@@ -100,7 +101,7 @@ struct DynGroup {
     keys.release(); keys_spare.release(); cand.release(); xbond.release(); adj_free.release(); free_end.release();
     hist[0].release(); hist[1].release(); hist_spare.release();
     hist32[0].release(); hist32[1].release(); hist32_spare.release();
-    adj_start.release(); adj_count.release(); adj_cursor.release(); p1_start.release(); adj.release();
+    adj_start.release(); adj_count.release(); adj_cursor.release(); p1_start.release(); p1_spare.release(); adj.release();
   }
 };
 
@@ -409,6 +410,7 @@ struct DemSim {
     for (auto& d : dyn) {
       build_adjacency(d.second.keys, d.second.m, d.second.adj_start, d.second.adj_count, d.second.adj_cursor,
                       d.second.p1_start, d.second.adj);
+      d.second.p1_n = n;
       if (handoff) mark_handoff(d.second);
     }
     for (auto& b : bond) build_adjacency(b.second.keys, b.second.nb, b.second.adj_start, b.second.adj_count,
@@ -621,8 +623,9 @@ struct DemSim {
     launch_scan(cell_count.p, cell_start.p, ncell + 1, scalars.p, scan_tmp.p, s);
     DEM_CUDA(cudaMemsetAsync(cell_cursor.p, 0, sizeof(int) * (ncell + 1), s));
     cell_list.reserve(std::max(n, 1));
-    launch_scatter_cells(P, cell_start.p, cell_cursor.p, cell_list.p, s);
-    launch_sort_cells(ncell, cell_start.p, cell_list.p, s);
+    scratch_i.reserve(n + 1);
+    launch_scatter_cells(P, cell_start.p, cell_cursor.p, scratch_i.p, s);
+    launch_place_cells(P, cell_start.p, scratch_i.p, cell_list.p, s);
     for (auto& b : bond) launch_bonds_rebuild(b.second.nb, b.second.ends.p, P.pflags, b.second.broken_step.p, s);
     timestamp++;
     c_rebuilds++;
@@ -644,11 +647,11 @@ struct DemSim {
   }
 
   void build_adjacency(DBuf<unsigned long long>& keys, int m, DBuf<int>& adj_start, DBuf<int>& adj_count,
-                       DBuf<int>& adj_cursor, DBuf<int>& p1_start, DBuf<int2>& adj) {
+                       DBuf<int>& adj_cursor, DBuf<int>& p1_start, DBuf<int2>& adj, bool have_p1 = false) {
     adj_start.reserve(n + 2); adj_count.reserve(n + 2); adj_cursor.reserve(n + 2); p1_start.reserve(n + 2);
     adj.grow(std::max(2 * m, 1));
     scan_tmp.reserve(scan_tmp_ints(n + 2));
-    launch_adj(keys.p, m, n, adj_count.p, p1_start.p, adj_start.p, adj_cursor.p, adj.p, scalars.p + 1, scan_tmp.p, s);
+    launch_adj(keys.p, m, n, adj_count.p, p1_start.p, adj_start.p, adj_cursor.p, adj.p, scalars.p + 1, scan_tmp.p, have_p1, s);
     c_launches += 5;
   }
 
@@ -657,23 +660,26 @@ struct DemSim {
   void dyn_full_update(DynGroup& G) {
     // with the device hand-off the list keeps the bond-excluded pairs (marked by mark_handoff)
     const ExclDev ex = handoff ? ExclDev{} : excl_of(G);
-    scratch_i.reserve(n + 1); scratch_j.reserve(n + 1);
+    scratch_i.reserve(n + 1); G.p1_spare.reserve(n + 2);
     launch_pairs_count(g, P, cur, cell_start.p, cell_list.p, ex, scratch_i.p, s);
     scan_tmp.reserve(scan_tmp_ints(n + 2));
-    launch_scan(scratch_i.p, scratch_j.p, n, scalars.p, scan_tmp.p, s);
+    launch_scan(scratch_i.p, G.p1_spare.p, n + 1, scalars.p, scan_tmp.p, s);
     const int m = read_int(scalars.p);
     c_launches += 3;
     check_list_size(m);
+    const int* old_p1 = G.p1_n == n ? G.p1_start.p : nullptr;
     G.keys_spare.grow(std::max(m, 1));
     if (G.kind != 0) G.hist_spare.grow(std::max(m, 1));
     if (fp32) {
       if (G.kind != 0) G.hist32_spare.grow(std::max(m, 1));
-      launch_pairs_write<float4>(g, P, cur, cell_start.p, cell_list.p, ex, scratch_j.p, G.keys_spare.p, hist_mode(G),
-                                 G.keys.p, G.m, G.hist32[cur].p, G.hist32_spare.p, s);
+      launch_pairs_write<float4>(g, P, cur, cell_start.p, cell_list.p, ex, G.p1_spare.p, G.keys_spare.p, hist_mode(G),
+                                 G.keys.p, G.m, old_p1, G.hist32[cur].p, G.hist32_spare.p, s);
     } else {
-      launch_pairs_write<double4>(g, P, cur, cell_start.p, cell_list.p, ex, scratch_j.p, G.keys_spare.p, hist_mode(G),
-                                  G.keys.p, G.m, G.hist[cur].p, G.hist_spare.p, s);
+      launch_pairs_write<double4>(g, P, cur, cell_start.p, cell_list.p, ex, G.p1_spare.p, G.keys_spare.p, hist_mode(G),
+                                  G.keys.p, G.m, old_p1, G.hist[cur].p, G.hist_spare.p, s);
     }
+    std::swap(G.p1_start, G.p1_spare);
+    G.p1_n = n;
     std::swap(G.keys, G.keys_spare);
     if (G.kind != 0) {
       if (fp32) {
@@ -685,7 +691,7 @@ struct DemSim {
       }
     }
     G.m = m;
-    build_adjacency(G.keys, m, G.adj_start, G.adj_count, G.adj_cursor, G.p1_start, G.adj);
+    build_adjacency(G.keys, m, G.adj_start, G.adj_count, G.adj_cursor, G.p1_start, G.adj, true);
     if (handoff) mark_handoff(G);
   }
 
@@ -764,6 +770,7 @@ struct DemSim {
       }
       G.m = m2;
       build_adjacency(G.keys, G.m, G.adj_start, G.adj_count, G.adj_cursor, G.p1_start, G.adj);
+      G.p1_n = n;
     }
     launch_clear_flags(n, P.flagged, s);  // getNewList clears every flag (ntable.hpp:658-662)
   }
@@ -2096,6 +2103,7 @@ struct DemSim {
       G.m = (int)rec.size();
       const int m = std::max(G.m, 1);
       G.keys.reserve(m);
+      G.p1_n = -1;
       for (int c = 0; c < 2; ++c) G.hist[c].reserve(m);
       if (fp32) for (int c = 0; c < 2; ++c) G.hist32[c].reserve(m);
       std::vector<unsigned long long> keys(G.m);
@@ -3055,6 +3063,7 @@ int dem_add_exclusion(dem_sim* h, const char* bonded, const char* dynamic) {
         if (G.kind != 0) DEM_CUDA(cudaMemcpyAsync(G.hist[s.cur].p, h2.data(), sizeof(double4) * G.m, cudaMemcpyHostToDevice, s.s));
       }
       s.build_adjacency(G.keys, G.m, G.adj_start, G.adj_count, G.adj_cursor, G.p1_start, G.adj);
+      G.p1_n = s.n;
       s.sync();
     }
     return DEM_OK;
