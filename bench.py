@@ -1136,8 +1136,9 @@ def main():
     achieved = alg_bytes / (step_ns * 1e-9) / 1e9
     peak, peak_kind = peaks()
     tpp_used = c1["threads_per_particle"]
-    kernel_name = (f"k_step<ROT=1, TPP={tpp_used}, FRIC, {'FP32' if args.precision == 32 else 'FP64'}>"
-                   if tpp_used != 16 else f"k_step_tiled<ROT=1, FRIC, {'FP32' if args.precision == 32 else 'FP64'}>")
+    # one lane without bonds: the multi-step kernel, whose time and bytes are given per timestep
+    form = {1: "k_run<ROT=1", 16: "k_step_tiled<ROT=1"}.get(tpp_used, f"k_step<ROT=1, TPP={tpp_used}")
+    kernel_name = f"{form}, FRIC, {'FP32' if args.precision == 32 else 'FP64'}>"
     traffic = traffic_per_launch()
     # the ncu capture's traffic counts only for the same kernel instance
     traffic_bytes = traffic["bytes_per_launch"] if traffic and traffic.get("kernel", "").startswith(kernel_name) else None

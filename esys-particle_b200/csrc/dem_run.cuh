@@ -26,6 +26,11 @@
 // each result goes to shared memory and the particle's own thread adds its entries in adjacency
 // order.  Every sum is then the one k_step forms with one lane per particle: the FP64 states are
 // bit-identical to its single-step launches.
+//
+// Measured (200 steps, a sheared cell of 250,000): 8.6 -> 4.6 ms in the FP32 form and 10.4 -> 4.9 ms in
+// FP64 against single-step launches; 31,000 particles, 100 steps: 2.0 -> 0.9 ms; 180 particles take
+// 2 us a step.  Bound by the chain of a step (L2 round trip, law, sums, grid barrier): at 250,000 in
+// FP64 24 % of the issue slots, 10 % of the FP64 pipe, 26 % of L2.
 #pragma once
 #include "dem_step.cuh"
 

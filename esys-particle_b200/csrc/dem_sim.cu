@@ -138,7 +138,9 @@ struct DemSim {
   int chunk = 0;         // steps launched per host round trip ("chunk"); 0 = kChunk, or kRunChunk in one multi-step launch
   static constexpr int kChunk = 64, kRunChunk = 1024;
   static constexpr double kRunDense = 4.5;  // mean entries from which an FP64 frictional packing takes single steps
-  static constexpr int kRunMin = 4;        // multi-step kernel without resident records: fewer steps go out singly
+  // multi-step kernel without resident records: fewer steps than this go out singly (its first prune costs
+  // some three steps; 250,000 particles in FP64: 3 steps 153 us in it and 142 singly, 4 steps 168 and 190)
+  static constexpr int kRunMin = 4;
   static constexpr int kRunEntries = 256;  // list entries per block that a small specimen's block count aims at
   // The multi-step kernel stays off until this neighbour search (counted by timestamp) after a launch
   // whose pruned lists did not fit; searches it is off for double while that goes on.
@@ -561,6 +563,8 @@ struct DemSim {
   // engine's latency for up to seven fields, one after another, was most of such a call.  Otherwise the
   // rows are packed on the device, then each wanted field is one copy into the caller's array
   // (direct DMA when the caller's memory is pinned).
+  // 8,000 rows take 99 us directly and 115 with the copies, 64,000 take 262 and 268; 125,000 and more
+  // are faster with the copies.
   static constexpr int kDirectRows = 1 << 16;
   int alive_n = -1;  // alive particles; -1: to be counted (only a neighbour search or a revival changes them)
   int get_particles(int* id, double* pos, double* vel, double* angvel, double* quat, double* force, double* moment) {

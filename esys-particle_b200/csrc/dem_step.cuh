@@ -337,8 +337,8 @@ __device__ __forceinline__ void pair_sums(const StepArgs& a, const ParticleBuf& 
       const DynDev& G = a.dyn[d];
       // Under the hand-off a particle none of whose bonds has failed walks its free entries only (its
       // held pairs' histories are zero in both buffers since the list was marked): on a bonded
-      // specimen eight of nine entries are held (240,000 bonded particles, FP32 form: a step of 116 us
-      // became 113; twelve specimens of 10,000 in one launch, 130 us at 8 lanes, now 4 and shorter).
+      // specimen eight of nine entries are held (240,000 bonded particles, FP32 form: a step of 120 us
+      // became 113 while few bonds have failed; twelve specimens of 10,000 in one launch, 130 us at 8 lanes, now 4 and shorter).
       const int e0 = __ldg(G.adj_start + i);
       const bool free_only = (FEAT & (F_BOND | F_BGATHER)) != 0 && G.adj_free && !flg;
       const int e1 = free_only ? __ldg(G.free_end + i) : __ldg(G.adj_start + i + 1);

@@ -277,9 +277,10 @@ int dem_wall_reactions_noalloc(int n, const double* particles, int nwall, const 
                                void* stream);
 
 /* Tuning knobs with no reference counterpart: "threads_per_particle" (0 = automatic: one lane for
- * a specimen with at least 768 particles per SM, else by the mean adjacency length; 1, 2, 4, 8;
+ * a specimen without bonds or with at least 768 particles per SM, else by the mean adjacency length,
+ * entries held by bonds under the hand-off left out; 1, 2, 4, 8 (2 and more: single-step launches);
  * 16 = block-cooperative tiles; 32 = warp-cooperative pair sums),
- * "chunk" (steps launched per host round trip), "store_forces" (keep per-particle F/M),
+ * "chunk" (steps launched per host round trip; automatic until set), "store_forces" (keep per-particle F/M),
  * "profile" (time the force/integration kernels with CUDA events), "precision" (64 = FP64 form,
  * 32 = FP32 pair forces with Kahan-compensated accumulation, FP64 positions / contact detection /
  * integration), "split" (1: pair kernel + integration kernel), "bond_pass" (1: each bond
