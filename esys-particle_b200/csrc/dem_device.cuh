@@ -99,9 +99,6 @@ struct DynDev {
   int scaling, meanR;
   const int* adj_start; // n+1
   const int2* adj;      // (partner slot, pair index | kAdjHeld | 0x80000000 when this particle is p1)
-  // device bond hand-off (else null): each particle's free entries, from adj_start[i] to free_end[i]
-  const int2* adj_free;
-  const int* free_end;  // n
   const double4* hist_in;   // RotFriction: Ffric xyz, w = slipping + 2*touching
   double4* hist_out;
   const float4* hist32_in;  // the same in the FP32 form

@@ -270,9 +270,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_pairs_write(Grid g, Particle
 
 // Device bond hand-off: for every pair of a freshly built list, the bond that excludes it
 // (an intact bond of an excluding group, TSubLattice::setExIG), (group << 28) | index, or -1.
-// A held pair's history is zeroed in both buffers of the form in use (the other's are null).
-__global__ void k_pairs_xbond(const unsigned long long* keys, int m, ExclDev ex, int* xbond, double4* h0, double4* h1,
-                              float4* f0, float4* f1) {
+__global__ void k_pairs_xbond(const unsigned long long* keys, int m, ExclDev ex, int* xbond) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m) return;
   const unsigned long long key = keys[k];
@@ -282,35 +280,22 @@ __global__ void k_pairs_xbond(const unsigned long long* keys, int m, ExclDev ex,
     if (p < ex.count[e] && ex.keys[e][p] == key && ex.broken_step[e][p] == kBondAlive) r = (ex.group[e] << 28) | p;
   }
   xbond[k] = r;
-  if (r < 0) return;
-  if (h0) h0[k] = h1[k] = make_double4(0.0, 0.0, 0.0, 0.0);
-  if (f0) f0[k] = f1[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
-void launch_pairs_xbond(const unsigned long long* keys, int m, const ExclDev& ex, int* xbond, double4* h0, double4* h1,
-                        float4* f0, float4* f1, cudaStream_t s) {
-  if (m > 0) k_pairs_xbond<<<(m + 255) / 256, 256, 0, s>>>(keys, m, ex, xbond, h0, h1, f0, f1);
+void launch_pairs_xbond(const unsigned long long* keys, int m, const ExclDev& ex, int* xbond, cudaStream_t s) {
+  if (m > 0) k_pairs_xbond<<<(m + 255) / 256, 256, 0, s>>>(keys, m, ex, xbond);
 }
 
 // Device bond hand-off: kAdjHeld on the adjacency entries of the pairs with an excluding bond,
-// so the step tests a bit of the entry it already holds instead of loading xbond; and each particle's
-// free entries, in their order, from the start of its range of adj_free to free_end.
-__global__ void k_adj_mark_held(int n, const int* xbond, const int* adj_start, int2* adj, int2* adj_free, int* free_end) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int e0 = adj_start[i], e1 = adj_start[i + 1];
-  int f = e0;
-  for (int e = e0; e < e1; ++e) {
-    int2 en = adj[e];
-    const bool held = xbond[en.y & kAdjIndex] >= 0;
-    en.y = (en.y & ~kAdjHeld) | (held ? kAdjHeld : 0);
-    adj[e] = en;
-    if (!held) adj_free[f++] = en;
-  }
-  free_end[i] = f;
+// so the step tests a bit of the entry it already holds instead of loading xbond.
+__global__ void k_adj_mark_held(int ne, const int* xbond, int2* adj) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  int2 en = adj[e];
+  en.y = (en.y & ~kAdjHeld) | (xbond[en.y & kAdjIndex] >= 0 ? kAdjHeld : 0);
+  adj[e] = en;
 }
-void launch_adj_mark_held(int n, const int* xbond, const int* adj_start, int2* adj, int2* adj_free, int* free_end,
-                          cudaStream_t s) {
-  if (n > 0) k_adj_mark_held<<<(n + 255) / 256, 256, 0, s>>>(n, xbond, adj_start, adj, adj_free, free_end);
+void launch_adj_mark_held(int ne, const int* xbond, int2* adj, cudaStream_t s) {
+  if (ne > 0) k_adj_mark_held<<<(ne + 255) / 256, 256, 0, s>>>(ne, xbond, adj);
 }
 
 // Wall candidates counted from the particles' flags; intact bonds counted from the break log.

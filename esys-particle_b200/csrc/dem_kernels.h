@@ -55,10 +55,8 @@ void launch_check_disp(const Particles& P, int cur, double half_alpha_sq, int* c
 void launch_move_tagged(const Particles& P, int cur, int tag, const double* d, cudaStream_t s);
 // idx: scratch of at least P.n ints (each servo thread's candidate list)
 void launch_wall_servo(const Particles& P, int cur, int w, WallDev* walls, const double* F, int* idx, cudaStream_t s);
-void launch_pairs_xbond(const unsigned long long* keys, int m, const ExclDev& ex, int* xbond, double4* h0, double4* h1,
-                        float4* f0, float4* f1, cudaStream_t s);
-void launch_adj_mark_held(int n, const int* xbond, const int* adj_start, int2* adj, int2* adj_free, int* free_end,
-                          cudaStream_t s);
+void launch_pairs_xbond(const unsigned long long* keys, int m, const ExclDev& ex, int* xbond, cudaStream_t s);
+void launch_adj_mark_held(int ne, const int* xbond, int2* adj, cudaStream_t s);
 void launch_count_candidates(int n, const unsigned* pflags, int* ncand, cudaStream_t s);
 void launch_particle_field(const Particles& P, int cur, int rot, int field, double* out, cudaStream_t s);
 void launch_particle_vector_field(const Particles& P, int cur, int field, const double* initpos, double* out,

@@ -93,12 +93,8 @@ struct DynGroup {
   int p1_n = -1;  // the particles that p1_start holds the list's ranges of; -1: not this list's
   DBuf<int2> adj;
   DBuf<int> xbond;  // device bond hand-off: excluding bond of each pair
-  DBuf<int2> adj_free;  // and each particle's free entries
-  DBuf<int> free_end;
-  int free_n = -1;     // the particles these are for
-  long long held = 0;  // the pairs held when the list was built (intact bonds of the excluding groups)
   void release() {
-    keys.release(); keys_spare.release(); cand.release(); xbond.release(); adj_free.release(); free_end.release();
+    keys.release(); keys_spare.release(); cand.release(); xbond.release();
     hist[0].release(); hist[1].release(); hist_spare.release();
     hist32[0].release(); hist32[1].release(); hist32_spare.release();
     adj_start.release(); adj_count.release(); adj_cursor.release(); p1_start.release(); p1_spare.release(); adj.release();
@@ -436,9 +432,8 @@ struct DemSim {
       for (int b = 0; b < 2; ++b) { G.hist[b].reserve(m); G.hist32[b].reserve(m); }
       launch_hist_convert(m, G.hist[cur].p, G.hist32[cur].p, want == 1, s);
     }
-    fp32 = want;
-    mark_handoff_all();
     sync();
+    fp32 = want;
   }
 
   // Precision check of the FP32-force form on the current state of an FP64 run:
@@ -704,37 +699,14 @@ struct DemSim {
     if (m > (long long)kAdjIndex + 1) throw StateError("a dynamic interaction group would hold more than 2^30 pairs");
   }
 
-  // Device bond hand-off: per pair of the list the intact bond that excludes it (xbond), kAdjHeld on
-  // the pair's two adjacency entries, the particles' free entries by themselves, and zero histories
-  // for the held pairs (the step writes none for them).  Run while the hand-off is on after every
-  // build of the group's adjacency and after every other write of its histories or bond states.
-  void mark_handoff(DynGroup& G, bool rebuilt = true) {
-    if (rebuilt) {
-      G.held = 0;
-      for (auto& x : G.excl) {
-        auto b = bond.find(x);
-        auto it = bond_alive.find(x);
-        if (b != bond.end()) G.held += it == bond_alive.end() ? b->second.nb : it->second;
-      }
-    }
+  // Device bond hand-off: per pair of the list the intact bond that excludes it (xbond) and
+  // kAdjHeld on the pair's two adjacency entries.  Run after every build of the group's
+  // adjacency while the hand-off is on.
+  void mark_handoff(DynGroup& G) {
     G.xbond.grow(std::max(G.m, 1));
-    G.adj_free.grow(std::max(2 * G.m, 1));
-    G.free_end.reserve(n + 1);
-    G.free_n = n;
-    double4* h[2] = {nullptr, nullptr};
-    float4* f[2] = {nullptr, nullptr};
-    if (G.kind != 0)
-      for (int c = 0; c < 2; ++c) {
-        if (fp32) { G.hist32[c].grow(std::max(G.m, 1)); f[c] = G.hist32[c].p; }
-        else { G.hist[c].grow(std::max(G.m, 1)); h[c] = G.hist[c].p; }
-      }
-    launch_pairs_xbond(G.keys.p, G.m, excl_of(G), G.xbond.p, h[0], h[1], f[0], f[1], s);
-    launch_adj_mark_held(n, G.xbond.p, G.adj_start.p, G.adj.p, G.adj_free.p, G.free_end.p, s);
+    launch_pairs_xbond(G.keys.p, G.m, excl_of(G), G.xbond.p, s);
+    launch_adj_mark_held(2 * G.m, G.xbond.p, G.adj.p, s);
     c_launches += 2;
-  }
-  void mark_handoff_all() {
-    if (handoff)
-      for (auto& d : dyn) if (d.second.adj_start.p) mark_handoff(d.second, false);
   }
 
   // PIS_NE / PIS_ED::update without a rebuild: append the "new list" of flagged pairs
@@ -946,8 +918,6 @@ struct DemSim {
       D.hist_in = G.hist[c].p; D.hist_out = G.hist[c ^ 1].p;
       D.hist32_in = G.hist32[c].p; D.hist32_out = G.hist32[c ^ 1].p;
       D.xbond = handoff ? G.xbond.p : nullptr;
-      D.adj_free = handoff && G.free_n == n ? G.adj_free.p : nullptr;
-      D.free_end = G.free_end.p;
     }
     a.nbond = 0;
     for (auto& b : bond) {
@@ -1057,29 +1027,19 @@ struct DemSim {
   // multi-step kernel's order of summation, whichever of the two takes a call.  With bonds, a
   // specimen with at least as many particles as the GPU keeps step threads resident (3 blocks of
   // 256 per SM) already fills it at one lane per particle, and a smaller one spreads each
-  // particle's adjacency over lanes by its mean length, held entries left out (a bonded block of 28,900
-  // particles under the hand-off, 40 steps: 3560, 2726, 2482, 2715 us at 1, 2, 4, 8 lanes; counted with
-  // the held entries it took 8).  The tiled kernels (kTiled) are chosen
+  // particle's adjacency over lanes by its mean length.  The tiled kernels (kTiled) are chosen
   // explicitly or by the ensemble autotuner.
   int pick_tpp() {
     if (tpp) return tpp == kTiled && !tiled_ok() ? 1 : tpp;
     if (bond.empty() || n >= 768LL * sms()) return 1;
-    const double mean = n ? (double)step_entries() / n : 0.0;
+    long long e = 0;
+    for (auto& d : dyn) e += 2LL * d.second.m;
+    for (auto& b : bond) e += 2LL * b.second.nb;
+    const double mean = n ? (double)e / n : 0.0;
     if (mean >= 12) return 8;
     if (mean >= 6) return 4;
     if (mean >= 2.5) return 2;
     return 1;
-  }
-
-  // Adjacency entries a step walks: the dynamic lists' less those held when the lists were built, and
-  // the bonds'.  Fixed between rebuilds, so a window's recomputed steps take its forward steps' lanes.
-  long long step_entries() const {
-    long long e = 0;
-    for (auto& d : dyn) {
-      e += 2LL * std::max(0LL, d.second.m - (handoff ? d.second.held : 0));
-    }
-    for (auto& b : bond) e += 2LL * b.second.nb;
-    return e;
   }
 
   // CLatticeMaster::runOneStep x nsteps (LatticeMaster.cpp:2602-2740), without savers and runnables.
@@ -1542,7 +1502,6 @@ struct DemSim {
     a.damp_iters = win.st_it.p + (size_t)j * 2 * n;
     a.store_forces = 0;
     a.replay = 1;
-    for (int d = 0; d < nd; ++d) a.dyn[d].adj_free = nullptr;  // the recompute's histories are written for every pair
     if (win.brk) a.pf_log = win.st_pf.p + (size_t)j * n;  // the wall candidacy this step used
     return a;
   }
@@ -2212,7 +2171,6 @@ struct DemSim {
     t = win.t0;
     DEM_CUDA(cudaMemcpyAsync(d_step, &t, sizeof(long long), cudaMemcpyHostToDevice, s));
     pending_ctrl = 0;
-    mark_handoff_all();
     sync();
     if (win.brk) refresh_counts();
     download_walls();
@@ -2314,7 +2272,8 @@ struct Ensemble {
     if (tpp) return tpp;
     long long e = 0, np = 0;
     for (DemSim* d : sims) {
-      e += d->step_entries();
+      for (auto& g : d->dyn) e += 2LL * g.second.m;
+      for (auto& b : d->bond) e += 2LL * b.second.nb;
       np += d->n;
     }
     const double mean = np ? (double)e / np : 0.0;
@@ -2591,7 +2550,6 @@ struct Ensemble {
       abase[k] = d.adj_begin(gR[k]);
       spec[k] = d.win_spec();
       h_args[k] = d.make_args(0);  // the recompute's base: live groups, walls, counters
-      for (int g = 0; g < h_args[k].ndyn; ++g) h_args[k].dyn[g].adj_free = nullptr;  // histories written for every pair
       ptile[k + 1] = ptile[k] + (d.n + 255) / 256;
       for (int b = 0; b < abase[k].nbond; ++b) {
         bptile[(size_t)k * kMaxBond + b + 1] = (abase[k].bond[b].nb + 127) / 128;
@@ -3208,8 +3166,6 @@ int dem_set_pair_states(dem_sim* h, const char* group, int n, const int* id1, co
       }
       ++done;
     }
-    s.mark_handoff_all();
-    s.sync();
     return done;
   });
 }

@@ -335,21 +335,14 @@ __device__ __forceinline__ void pair_sums(const StepArgs& a, const ParticleBuf& 
     const bool flg = handoff_flag<FEAT>(a, i);
     for (int d = 0; d < a.ndyn; ++d) {
       const DynDev& G = a.dyn[d];
-      // Under the hand-off a particle none of whose bonds has failed walks its free entries only (its
-      // held pairs' histories are zero in both buffers since the list was marked): on a bonded
-      // specimen eight of nine entries are held (240,000 bonded particles, FP32 form: a step of 120 us
-      // became 113 while few bonds have failed; twelve specimens of 10,000 in one launch, 130 us at 8 lanes, now 4 and shorter).
-      const int e0 = __ldg(G.adj_start + i);
-      const bool free_only = (FEAT & (F_BOND | F_BGATHER)) != 0 && G.adj_free && !flg;
-      const int e1 = free_only ? __ldg(G.free_end + i) : __ldg(G.adj_start + i + 1);
-      const int2* adj = free_only ? G.adj_free : G.adj;
+      const int e0 = __ldg(G.adj_start + i), e1 = __ldg(G.adj_start + i + 1);
       for (int e = e0 + lane; e < e1; e += TPP * kBatch) {
         int2 en[kBatch];
         double4 pjs[kBatch];
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
           const int eb = e + b * TPP;
-          en[b] = eb < e1 ? __ldg(adj + eb) : make_int2(-1, 0);
+          en[b] = eb < e1 ? __ldg(G.adj + eb) : make_int2(-1, 0);
         }
         // device bond hand-off: a pair is skipped while the bond that excluded it holds, and its
         // partner record is not fetched

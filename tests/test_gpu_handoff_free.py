@@ -1,10 +1,9 @@
-"""Free adjacency entries under the device bond hand-off: a particle none of whose bonds has failed
-walks only the entries that no bond holds, dealt to its lanes as the host hand-off's list is.
+"""Device bond hand-off against the host hand-off, whose lists leave the held pairs out, at each
+number of lanes while no bond fails, and at one lane across failures with a change of the precision
+form and back in between (which rounds both sides' histories alike).
 
-Bar: bit equality with the host hand-off, whose lists leave the held pairs out, at each number of
-lanes while no bond fails; and at one lane also across failures with the lists marked anew in
-between (a change of precision and back, which rounds both sides' histories alike).
-All tests need a GPU.
+Bar: bit equality.  At several lanes it holds because the block's only contacts are its bonds and
+the platens: the held entries contribute nothing, wherever they fall.  All tests need a GPU.
 """
 import numpy as np
 import pytest
@@ -46,7 +45,7 @@ def test_no_failures_equal_host_handoff(dem_lib, precision, tpp):
 
 
 @pytest.mark.parametrize("precision", [64, 32])
-def test_lists_marked_anew_between_failures(dem_lib, precision):
+def test_change_of_form_between_failures(dem_lib, precision):
     host, dev = _both(dem_lib, precision, 1, (0.3, 0.6, 0.6, 0.3))
     for s in (host, dev):
         S.run_loaded(s, 100, 0.002)
