@@ -198,6 +198,7 @@ struct StepArgs {
 
 // Launch of the multi-step kernel (dem_run.cuh).
 constexpr int kRunThreads = 512;
+constexpr size_t kRunSmem = 220 * 1024;  // the most a block takes: of its 227 KB, less the kernel's static arrays
 struct RunArgs {
   int nsteps;     // timesteps of this launch
   int blocks;     // at most one per SM

@@ -655,7 +655,8 @@ inline cudaError_t launch_run_as(const StepArgs& a, RunArgs ra, cudaStream_t s) 
   const void* fn = reinterpret_cast<const void*>(k_run<R, FEAT, FP32, ONE>);
   using Smem = RunSmem<R, FEAT, FP32, ONE>;
   const size_t smem = run_layout(R, Smem::FRIC, Smem::MOM, FP32, ONE, ra.ppb, ra.pool, ra.room).bytes;
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the attribute is the function's, not the launch's: every handle and host thread sets the same value
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
   if (e != cudaSuccess) return e;
   StepArgs arg = a;
   void* p[] = {&arg, &ra};

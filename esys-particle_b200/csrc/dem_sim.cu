@@ -1000,13 +1000,12 @@ struct DemSim {
     ra.ppb = ra.chunk * ((groups + ra.blocks - 1) / ra.blocks);
     ra.half = (float)(alpha / 16);
     ra.horizon = 64.f;
-    constexpr size_t kSmem = 220 * 1024;  // of a block's 227 KB, less the kernel's static arrays
     // every entry of the list in shared memory, results included, beside the particles' records
     const long long worst = std::max(64LL, (long long)std::ceil(1.25 * mean * ra.ppb));
     ra.one = 1;
     if (worst < 65536) {
       ra.pool = ra.room = (int)worst;
-      if (run_layout(rot, fric, moment, fp32, true, ra.ppb, ra.pool, ra.room).bytes <= kSmem) return true;
+      if (run_layout(rot, fric, moment, fp32, true, ra.ppb, ra.pool, ra.room).bytes <= kRunSmem) return true;
     }
     // else the records stay in L2, and what is left is shared 60:40 between entries and results
     ra.one = 0;
@@ -1016,8 +1015,8 @@ struct DemSim {
     // 1718 here, 2893 singly; in the FP32 form the former take 1018 and 1155).
     if (!fp32 && fric && mean >= kRunDense) return false;
     const size_t fixed = run_layout(rot, fric, moment, fp32, false, ra.ppb, 0, 0).bytes + 128;
-    if (ra.ppb > 65535 || fixed > kSmem / 2) return false;
-    const size_t left = kSmem - fixed, res = (size_t)(fp32 ? 4 : 8) * (moment ? 9 : (fric ? 6 : 3));
+    if (ra.ppb > 65535 || fixed > kRunSmem / 2) return false;
+    const size_t left = kRunSmem - fixed, res = (size_t)(fp32 ? 4 : 8) * (moment ? 9 : (fric ? 6 : 3));
     ra.pool = (int)std::min<size_t>(std::min<long long>(worst, 65535), left * 6 / 10 / 34);
     ra.room = (int)std::min<size_t>(ra.pool, (left - (size_t)34 * ra.pool) / res);
     return ra.room >= 1024 && ra.pool >= ra.ppb / 4;

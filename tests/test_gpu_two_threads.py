@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", [64, 32])
 def test_small_and_large_specimen_side_by_side(dem_lib, precision):
-    """Launches of one kernel with unlike shares of a block's shared memory (33 KB and 130 KB or so)."""
+    """Launches of one kernel with unlike shares of a block's shared memory."""
     from esys.lsm import _capi
 
     def build(n):
