@@ -10,8 +10,11 @@
 // host round trip; a step that needs host work (rebuild, bond-break update)
 // raises a control flag that makes the remaining launches of the chunk
 // return at once, and the host resumes from there.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
@@ -542,15 +545,35 @@ struct DemSim {
     return 0;
   }
 
-  // The device address of page-locked host memory, or null for any other.
+  // The device address of `count` elements of page-locked host memory that a kernel may write, or null
+  // for any other: pageable or managed memory, an address that is no multiple of the element's size
+  // (rows behind a header; a copy takes any address), an array that its page-locked range does not hold whole.
   template <class T>
-  static T* mapped(T* host) {
+  static T* mapped(T* host, size_t count) {
+    if (reinterpret_cast<uintptr_t>(host) % sizeof(T)) return nullptr;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
       (void)cudaGetLastError();
       return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? static_cast<T*>(at.devicePointer) : nullptr;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+    using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+      void* f = nullptr;
+      if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault) != cudaSuccess) {
+        (void)cudaGetLastError();
+        f = nullptr;
+      }
+      return reinterpret_cast<Query>(f);
+    }();
+    const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (!query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) != CUDA_SUCCESS)
+      return nullptr;
+    const size_t before = (size_t)(p - start), bytes = count * sizeof(T);
+    return p >= start && before <= size && bytes <= size - before ? static_cast<T*>(at.devicePointer) : nullptr;
   }
 
   // The alive particles in slot order into the caller's host arrays (each may be null).  A specimen
@@ -579,8 +602,8 @@ struct DemSim {
       double* const want[6] = {pos, vel, angvel, quat, force, moment};
       bool all = true;
       for (int f = 0; f < 6 && all; ++f)
-        if (want[f]) all = (to.field[f] = mapped(want[f])) != nullptr;
-      if (id && all) all = (to.id = mapped(id)) != nullptr;
+        if (want[f]) all = (to.field[f] = mapped(want[f], (size_t)n * (f == 3 ? 4 : 3))) != nullptr;
+      if (id && all) all = (to.id = mapped(id, (size_t)n)) != nullptr;
       if (all) {
         launch_rows_direct(P, cur, rot, to, s);
         DEM_CUDA(cudaGetLastError());
@@ -3322,6 +3345,9 @@ int dem_precision_report(dem_sim* h, double* out, int n) {
     return std::min(n, 7);
   });
 }
+
+// Whether `count` doubles at `host` are written by a kernel in dem_get_particles (the rule alone, for tests).
+int dem_rows_mapped(double* host, size_t count) { return DemSim::mapped(host, count) != nullptr; }
 
 int dem_set_option(dem_sim* h, const char* key, double value) {
   return guard(h, [&](DemSim& s) {
