@@ -209,6 +209,7 @@ struct RunArgs {
   int room;       // entries whose results it can hold at a time
   float half;     // least allowance of movement of the first prune
   float horizon;  // steps whose movement at the particle's speed its allowance covers
+  int polls;      // polls after which a wait at the grid barrier gives up
 };
 // Shared memory of one of its blocks: byte offsets of the arrays and the total.
 struct RunLayout {

@@ -36,7 +36,6 @@
 
 namespace dem {
 
-constexpr int kRunPolls = 1 << 24;     // polls of a grid barrier before it gives up (seconds)
 constexpr int kRunPruneSteps = 8;      // prunes closer than this many steps double the allowances
 enum : int { RUN_STOP = 1, RUN_PRUNE = 2, RUN_LOST = 4 };
 
@@ -48,6 +47,7 @@ enum : int { RUN_STOP = 1, RUN_PRUNE = 2, RUN_LOST = 4 };
 struct RunBarrier {
   unsigned long long* word;  // [2]
   unsigned nblocks;
+  int polls;
   int k = 0;
   unsigned seen[2] = {0u, 0u};  // upper halves
   // Arrival with this block's requests; one thread, after a __syncthreads.
@@ -63,7 +63,7 @@ struct RunBarrier {
     const unsigned target = (unsigned)((k >> 1) + 1) * nblocks;
     const int w = k & 1;
     ++k;
-    for (int it = 0; it < kRunPolls; ++it) {
+    for (int it = 0; it < polls; ++it) {
       unsigned long long v;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word + w) : "memory");
       if ((unsigned)v >= target) {
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) k_run(const StepArgs a, const 
     return fminf(allow_max, fmaxf(half, reach_t * sqrtf(vx * vx + vy * vy + vz * vz)));
   };
   const int lanes = ppb <= kRunThreads / 4 ? 8 : 4;  // per particle in a prune
-  RunBarrier barrier{a.run_word, nb};  // used by kBarrierThread
+  RunBarrier barrier{a.run_word, nb, ra.polls};  // used by kBarrierThread
   int ran = 0, pruned_at = 0, used = 0, full = 0;
   bool prune = true;
   while (true) {

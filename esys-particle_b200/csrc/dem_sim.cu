@@ -144,6 +144,12 @@ struct DemSim {
   // The multi-step kernel stays off until this neighbour search (counted by timestamp) after a launch
   // whose pruned lists did not fit; searches it is off for double while that goes on.
   int run_off_until = -1, run_backoff = 1;
+  int run_polls = 1 << 24;  // "barrier_polls": of a wait at its grid barrier before it gives up (seconds)
+  // Set when a wait gave up: the blocks may stand at different steps, so the state is no timestep's and
+  // every later call on the handle is refused.
+  bool lost = false;
+  static constexpr const char* kLostText =
+      "the state was lost when a grid barrier of the multi-step kernel timed out; destroy this handle";
   int store_forces = 1;
   int fp32 = 0;          // 1 = FP32-force / FP64-integration form
   int split = -1;        // -1 automatic, 0 fused step kernel, 1 pair kernel + integration kernel
@@ -1023,6 +1029,7 @@ struct DemSim {
     ra.ppb = ra.chunk * ((groups + ra.blocks - 1) / ra.blocks);
     ra.half = (float)(alpha / 16);
     ra.horizon = 64.f;
+    ra.polls = run_polls;
     // every entry of the list in shared memory, results included, beside the particles' records
     const long long worst = std::max(64LL, (long long)std::ceil(1.25 * mean * ra.ppb));
     ra.one = 1;
@@ -1134,6 +1141,7 @@ struct DemSim {
       const int ran = (int)(dev_t - t0);
       pending_ctrl = h_ctrl[2];
       if (pending_ctrl & CTRL_LOST) {
+        lost = true;
         err = "a grid barrier of the multi-step kernel timed out";
         return -3;
       }
@@ -2210,6 +2218,11 @@ struct DemSim {
 struct Ensemble {
   std::string err;
   std::vector<DemSim*> sims;
+  Ensemble& usable() {
+    for (DemSim* d : sims)
+      if (d->lost) throw StateError(DemSim::kLostText);
+    return *this;
+  }
   std::vector<cudaStream_t> saved;
   cudaStream_t s = nullptr;
   int tpp = 0, chunk = 64, use_graph = 1, profile = 0;
@@ -2697,6 +2710,7 @@ int guard(dem_sim* h, F&& f) {
   if (!s) return DEM_ERR_ARG;
   (void)cudaGetLastError();  // every runtime call is checked where it is made; drop a reported, non-sticky error
   try {
+    if (s->lost) throw dem::StateError(DemSim::kLostText);
     return f(*s);
   } catch (const dem::CudaError& e) {
     s->err = e.what();
@@ -3378,6 +3392,10 @@ int dem_set_option(dem_sim* h, const char* key, double value) {
       s.adj_tangents = v;
     } else if (k == "adjoint_pair_duals") {
       s.adj_pair_duals = value != 0;
+    } else if (k == "barrier_polls") {
+      if (!(value >= 0 && value <= 1 << 30) || value != std::floor(value))
+        throw std::invalid_argument("barrier_polls must be a whole number in [0, 2^30]");
+      s.run_polls = (int)value;
     } else if (k == "event_capacity") {
       if (!(value >= 0 && value <= 1 << 30) || value != std::floor(value))
         throw std::invalid_argument("event_capacity must be a whole number in [0, 2^30] (0 = one entry per bond)");
@@ -3662,16 +3680,16 @@ int eguard(dem_ensemble* h, F&& f) {
 extern "C" {
 
 int dem_ensemble_step(dem_ensemble* h, int nsteps) {
-  return eguard(h, [&](dem::Ensemble& e) { return e.step(nsteps); });
+  return eguard(h, [&](dem::Ensemble& e) { return e.usable().step(nsteps); });
 }
 
 int dem_ensemble_window_forward(dem_ensemble* h, int nsteps, int checkpoint_every, double* const* reactions) {
-  return eguard(h, [&](dem::Ensemble& e) { return e.window_forward(nsteps, checkpoint_every, reactions); });
+  return eguard(h, [&](dem::Ensemble& e) { return e.usable().window_forward(nsteps, checkpoint_every, reactions); });
 }
 
 int dem_ensemble_window_adjoint(dem_ensemble* h, const double* const* grad_reactions, double* const* grad_params,
                                 double* const* grad_vel, double* const* grad_angvel) {
-  return eguard(h, [&](dem::Ensemble& e) { return e.window_adjoint(grad_reactions, grad_params, grad_vel, grad_angvel); });
+  return eguard(h, [&](dem::Ensemble& e) { return e.usable().window_adjoint(grad_reactions, grad_params, grad_vel, grad_angvel); });
 }
 
 int dem_ensemble_set_option(dem_ensemble* h, const char* key, double value) {

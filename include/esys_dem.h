@@ -277,9 +277,8 @@ int dem_wall_reactions_noalloc(int n, const double* particles, int nwall, const 
                                void* stream);
 
 /* Tuning knobs with no reference counterpart: "threads_per_particle" (0 = automatic: one lane for
- * a specimen without bonds or with at least 768 particles per SM, else by the mean adjacency length,
- * entries held by bonds under the hand-off left out; 1, 2, 4, 8 (2 and more: single-step launches);
- * 16 = block-cooperative tiles; 32 = warp-cooperative pair sums),
+ * a specimen without bonds or with at least 768 particles per SM, else by the mean adjacency length;
+ * 1, 2, 4, 8 (2 and more: single-step launches); 16 = block-cooperative tiles; 32 = warp-cooperative pair sums),
  * "chunk" (steps launched per host round trip; automatic until set), "store_forces" (keep per-particle F/M),
  * "profile" (time the force/integration kernels with CUDA events), "precision" (64 = FP64 form,
  * 32 = FP32 pair forces with Kahan-compensated accumulation, FP64 positions / contact detection /
@@ -292,7 +291,10 @@ int dem_wall_reactions_noalloc(int n, const double* particles, int nwall, const 
  * smaller log that fills makes the dem_step or dem_ensemble_step call in which it filled return
  * DEM_ERR_OVERFLOW after running all its steps; the bond states stay exact, dem_get_breaks holds
  * the events logged before it filled, later calls go on, and the capacity of a group whose log
- * overflowed can no longer change). */
+ * overflowed can no longer change),
+ * "barrier_polls" (polls after which a wait of the multi-step kernel's blocks for one another gives up,
+ * 2^24 at first, some seconds; dem_step then returns DEM_ERR_CUDA and every later call DEM_ERR_STATE:
+ * the state is no timestep's any more). */
 int dem_set_option(dem_sim* h, const char* key, double value);
 
 /* ---- Field savers ----------------------------------------------------------------------- */

@@ -90,3 +90,24 @@ def test_fp32_form_equals_single_steps(gpu, kw, steps):
         assert np.abs(pa[k] - pb[k]).max() <= 1e-5 * np.abs(pb[k]).max(), k
     for x, y in zip(a.pairs("friction")[:2], b.pairs("friction")[:2]):
         assert np.array_equal(x, y)
+
+
+def test_a_barrier_that_gives_up_loses_the_handle(gpu):
+    """A wait that runs out (here at once: no poll at all) ends the launch with blocks at unlike steps.
+    The call reports it and the handle refuses everything that follows; others are unaffected."""
+    from esys.lsm._capi import DemError, Ensemble
+
+    s, other = (S.friction_pack(gpu, nx=13, ny=11, nz=12) for _ in range(2))
+    for x in (s, other):
+        x.step(3)
+    s.set_option("barrier_polls", 0)
+    with pytest.raises(DemError, match="timed out"):
+        s.step(5)
+    e = Ensemble([s, other])
+    for call in (lambda: s.step(1), s.particles, lambda: s.wall("roof"), lambda: s.set_particles(vel=np.zeros((1, 3))),
+                 lambda: s.window_forward(2, 2), lambda: s.set_option("precision", 32), lambda: e.step(1)):
+        with pytest.raises(DemError, match="state was lost"):
+            call()
+    e.close()
+    other.step(5)
+    assert other.timestep == 8
