@@ -145,6 +145,8 @@ struct DemSim {
   // whose pruned lists did not fit; searches it is off for double while that goes on.
   int run_off_until = -1, run_backoff = 1;
   int run_polls = 1 << 24;  // "barrier_polls": of a wait at its grid barrier before it gives up (seconds)
+  int run_blocks = 0;       // "run_blocks": its blocks; 0 = one per SM, fewer for a small specimen
+  bool run_refused = false; // the GPU cannot hold that many at once: single steps from then on
   // Set when a wait gave up: the blocks may stand at different steps, so the state is no timestep's and
   // every later call on the handle is refused.
   bool lost = false;
@@ -1010,9 +1012,10 @@ struct DemSim {
 
   // The multi-step kernel's launch (dem_run.cuh); false where dem_step takes single-step launches:
   // with bonds, the lane, tiled and warp-cooperative forms chosen by the caller, a specimen whose
-  // particles alone fill a block's shared memory, or one whose pruned lists did not fit lately.
+  // particles alone fill a block's shared memory, one whose pruned lists did not fit lately, or where
+  // the GPU cannot hold all its blocks at once (a process that may use some of its SMs only).
   bool run_shape(RunArgs& ra) {
-    if (!bond.empty() || split == 1 || tpp > 1 || n < 1 || timestamp < run_off_until) return false;
+    if (!bond.empty() || split == 1 || tpp > 1 || n < 1 || run_refused || timestamp < run_off_until) return false;
     bool fric = false, moment = false;
     long long m2 = 0;
     for (auto& d : dyn) {
@@ -1023,7 +1026,7 @@ struct DemSim {
     const double mean = (double)m2 / n;
     // one block per SM; a small specimen takes fewer blocks, of kRunEntries entries or so
     const double want = n * std::max(mean, 1.0) / kRunEntries;
-    ra.blocks = (int)std::min<double>(sms(), std::max(1.0, std::ceil(want)));
+    ra.blocks = run_blocks > 0 ? run_blocks : (int)std::min<double>(sms(), std::max(1.0, std::ceil(want)));
     ra.chunk = n >= 256LL * ra.blocks ? 32 : (n >= 8LL * ra.blocks ? 8 : 1);
     const int groups = (n + ra.chunk - 1) / ra.chunk;
     ra.ppb = ra.chunk * ((groups + ra.blocks - 1) / ra.blocks);
@@ -1106,7 +1109,7 @@ struct DemSim {
       const bool multi = run_shape(ra) && (ra.one || nsteps - done >= kRunMin);
       const int k = std::min(multi ? std::min(chunk > 0 ? chunk : kRunChunk, kRunChunk) : (chunk > 0 ? chunk : kChunk),
                              nsteps - done);
-      const int grid = std::max(step_grid(n, t_pp), sms());  // partials of either kernel's blocks
+      const int grid = std::max(step_grid(n, t_pp), multi ? ra.blocks : 0);  // partials of the kernel's blocks
       d_wall_partial.reserve((size_t)grid * kMaxWalls * 3);
       clear_control();
       const long long t0 = t;
@@ -1121,7 +1124,13 @@ struct DemSim {
         StepArgs a = make_args(cur);
         a.force_step = t_last;
         ra.nsteps = k;
-        DEM_CUDA(fp32 ? launch_run_fp32(a, rot != 0, ra, s) : launch_run(a, rot != 0, ra, s));
+        const cudaError_t e = fp32 ? launch_run_fp32(a, rot != 0, ra, s) : launch_run(a, rot != 0, ra, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+          (void)cudaGetLastError();
+          run_refused = true;
+          continue;
+        }
+        DEM_CUDA(e);
       } else {
         for (int j = 0; j < k; ++j) {
           StepArgs a = make_args((cur + j) & 1);
@@ -3396,6 +3405,11 @@ int dem_set_option(dem_sim* h, const char* key, double value) {
       if (!(value >= 0 && value <= 1 << 30) || value != std::floor(value))
         throw std::invalid_argument("barrier_polls must be a whole number in [0, 2^30]");
       s.run_polls = (int)value;
+    } else if (k == "run_blocks") {
+      if (!(value >= 0 && value <= 65535) || value != std::floor(value))
+        throw std::invalid_argument("run_blocks must be a whole number in [0, 65535]");
+      s.run_blocks = (int)value;
+      s.run_refused = false;
     } else if (k == "event_capacity") {
       if (!(value >= 0 && value <= 1 << 30) || value != std::floor(value))
         throw std::invalid_argument("event_capacity must be a whole number in [0, 2^30] (0 = one entry per bond)");

@@ -292,7 +292,8 @@ int dem_wall_reactions_noalloc(int n, const double* particles, int nwall, const 
  * DEM_ERR_OVERFLOW after running all its steps; the bond states stay exact, dem_get_breaks holds
  * the events logged before it filled, later calls go on, and the capacity of a group whose log
  * overflowed can no longer change),
- * "barrier_polls" (polls after which a wait of the multi-step kernel's blocks for one another gives up,
+ * "run_blocks" (blocks of the multi-step kernel, at most 65535; 0: one per SM, fewer for a small specimen;
+ * where the GPU cannot hold them all at once the specimen takes single steps), "barrier_polls" (polls after which a wait of the multi-step kernel's blocks for one another gives up,
  * 2^24 at first, some seconds; dem_step then returns DEM_ERR_CUDA and every later call DEM_ERR_STATE:
  * the state is no timestep's any more). */
 int dem_set_option(dem_sim* h, const char* key, double value);

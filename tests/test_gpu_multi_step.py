@@ -111,3 +111,19 @@ def test_a_barrier_that_gives_up_loses_the_handle(gpu):
     e.close()
     other.step(5)
     assert other.timestep == 8
+
+
+@pytest.mark.parametrize("blocks,launches", [(11, 1), (37, 1), (65535, 10)])
+def test_number_of_blocks(gpu, blocks, launches):
+    """Any number of blocks that the GPU holds at once gives the same states; more than that is refused
+    by the launch and the call goes on in single steps (as where a process may use a part of the GPU)."""
+    a, b = (S.friction_pack(gpu, nx=13, ny=11, nz=12) for _ in range(2))
+    a.set_option("run_blocks", blocks)
+    b.set_option("split", 1)
+    for s in (a, b):
+        s.step(2)
+    before = a.counters()["launches"]
+    for s in (a, b):
+        s.step(10)
+    assert a.counters()["launches"] - before == launches
+    _equal(a, b, ["friction"], ["floor", "roof"])
