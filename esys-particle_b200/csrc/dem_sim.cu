@@ -137,9 +137,13 @@ struct DemSim {
   int chunk = 0;         // steps launched per host round trip ("chunk"); 0 = kChunk, or kRunChunk in one multi-step launch
   static constexpr int kChunk = 64, kRunChunk = 1024;
   static constexpr double kRunDense = 4.5;  // mean entries from which an FP64 frictional packing takes single steps
-  // multi-step kernel without resident records: fewer steps than this go out singly (its first prune costs
-  // some three steps; 250,000 particles in FP64: 3 steps 153 us in it and 142 singly, 4 steps 168 and 190)
-  static constexpr int kRunMin = 4;
+  // Fewest steps of a call that the multi-step kernel takes: its launch, first prune and barriers cost as
+  // much as one to three steps.  Frictional packings in FP64, us a call there and in single launches:
+  //   resident records, 6,859:  one step 44 / 41, two 42 / 59;  13,824:  one 44 / 41, two 47 / 59
+  //   32,768 (224 a block):     one 53 / 41, two 67 / 61, three 77 / 85
+  //   records in L2, 250,000:   three 153 / 142, four 168 / 190
+  static constexpr int kRunMinBlock = 192;  // particles a block up to which two resident steps gain
+  static int run_min(const RunArgs& ra) { return ra.one ? (ra.ppb <= kRunMinBlock ? 2 : 3) : 4; }
   static constexpr int kRunEntries = 256;  // list entries per block that a small specimen's block count aims at
   // The multi-step kernel stays off until this neighbour search (counted by timestamp) after a launch
   // whose pruned lists did not fit; searches it is off for double while that goes on.
@@ -1106,7 +1110,7 @@ struct DemSim {
       // launch a chunk of force + integration steps
       const int t_pp = pick_tpp();
       RunArgs ra{};
-      const bool multi = run_shape(ra) && (ra.one || nsteps - done >= kRunMin);
+      const bool multi = run_shape(ra) && nsteps - done >= run_min(ra);
       const int k = std::min(multi ? std::min(chunk > 0 ? chunk : kRunChunk, kRunChunk) : (chunk > 0 ? chunk : kChunk),
                              nsteps - done);
       const int grid = std::max(step_grid(n, t_pp), multi ? ra.blocks : 0);  // partials of the kernel's blocks

@@ -127,3 +127,21 @@ def test_number_of_blocks(gpu, blocks, launches):
         s.step(10)
     assert a.counters()["launches"] - before == launches
     _equal(a, b, ["friction"], ["floor", "roof"])
+
+
+@pytest.mark.parametrize("shape,squeeze,launches", [((13, 11, 12), 0.93, (1, 1, 1, 1)), ((32, 32, 32), 1.04, (1, 2, 1, 1)),
+                                                    ((42, 40, 40), 1.14, (1, 2, 3, 1))])
+def test_short_calls(gpu, shape, squeeze, launches):
+    """Calls of one to four steps: singly where the multi-step kernel's first prune costs more than the
+    launches it saves (few and many particles a block, records in L2), and the same states."""
+    kw = dict(zip(("nx", "ny", "nz"), shape), squeeze=squeeze)
+    a, b = (S.friction_pack(gpu, **kw) for _ in range(2))
+    b.set_option("split", 1)
+    for s in (a, b):
+        s.step(1)
+    for k, want in zip((1, 2, 3, 4), launches):
+        before = a.counters()["launches"]
+        a.step(k)
+        assert a.counters()["launches"] - before == want, k
+        b.step(k)
+    _equal(a, b, ["friction"], ["floor", "roof"])
