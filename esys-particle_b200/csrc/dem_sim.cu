@@ -202,8 +202,8 @@ struct DemSim {
   int *d_ctrl = nullptr, *d_stop = nullptr;
   unsigned long long* d_run = nullptr;
   int num_sms = 0;       // of the current device; 0 until asked for
-  int* h_ctrl = nullptr;  // pinned
-  double* h_walls = nullptr;  // pinned: the wall groups' origins and reactions (6 each) as a kernel writes them
+  int* h_ctrl = nullptr;  // pinned, one allocation of a handle
+  double* h_walls = nullptr;  // its second part: the wall groups' origins and reactions (6 each) as a kernel writes them
   long long t = 0;
   int timestamp = 0, last_ns = -1;
   bool first = true;
@@ -223,8 +223,8 @@ struct DemSim {
 
   DemSim() {
     DEM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    DEM_CUDA(cudaMallocHost(&h_ctrl, 4 * sizeof(long long)));
-    DEM_CUDA(cudaMallocHost(&h_walls, 6 * kMaxWalls * sizeof(double)));
+    DEM_CUDA(cudaMallocHost(&h_ctrl, 4 * sizeof(long long) + 6 * kMaxWalls * sizeof(double)));
+    h_walls = reinterpret_cast<double*>(h_ctrl) + 4;
     d_block_counter.reserve(1); d_ctl.reserve(4); scalars.reserve(8);
     d_step = d_ctl.p;
     d_ctrl = reinterpret_cast<int*>(d_ctl.p + 1);
@@ -252,7 +252,6 @@ struct DemSim {
     stage.release(); stage_slot.release(); scratch_d.release(); sig.release(); d_servo_idx.release(); d_brk.release(); rows.release(); pack_id.release();
     pack.release();
     if (h_ctrl) cudaFreeHost(h_ctrl);
-    if (h_walls) cudaFreeHost(h_walls);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (own_stream) cudaStreamDestroy(s);
