@@ -211,6 +211,7 @@ struct DemSim {
   bool own_stream = true;
   // counters (dem_get_counters)
   long long c_steps = 0, c_contacts = 0, c_rebuilds = 0, c_launches = 0, prof_steps = 0;
+  long long c_runs = 0, c_runs_full = 0;  // launches of the multi-step kernel; those that its lists did not fit
   double prof_ms = 0.0;
   bool profile = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1146,6 +1147,7 @@ struct DemSim {
       }
       if (profile) DEM_CUDA(cudaEventRecord(ev1, s));
       c_launches += multi ? 1 : (two ? 2LL * k : k);
+      c_runs += multi;
       DEM_CUDA(cudaMemcpyAsync(h_ctrl, d_ctl.p, 2 * sizeof(long long), cudaMemcpyDeviceToHost, s));  // counter, bits
       sync();
       long long dev_t;
@@ -1161,6 +1163,7 @@ struct DemSim {
         run_off_until = timestamp + run_backoff;
         run_backoff = std::min(64, 2 * run_backoff);
         pending_ctrl &= ~CTRL_FULL;
+        c_runs_full += 1;
         if (ran == 0) continue;
       } else if (multi) {
         run_backoff = 1;
@@ -3334,11 +3337,11 @@ int dem_set_stream(dem_sim* h, void* stream) {
 int dem_get_counters(dem_sim* h, long long* out, int n) {
   return guard(h, [&](DemSim& s) {
     const long long search_due = (s.first || (s.pending_ctrl & dem::CTRL_REBUILD)) ? 1 : 0;
-    long long v[9] = {s.c_steps, s.c_contacts, s.c_rebuilds, s.c_launches,
+    long long v[11] = {s.c_steps, s.c_contacts, s.c_rebuilds, s.c_launches,
                       (long long)(s.prof_ms * 1e6), s.prof_steps, s.contacts_per_step(), (long long)s.pick_tpp(),
-                      search_due};
-    for (int i = 0; i < n && i < 9; ++i) out[i] = v[i];
-    return std::min(n, 9);
+                      search_due, s.c_runs, s.c_runs_full};
+    for (int i = 0; i < n && i < 11; ++i) out[i] = v[i];
+    return std::min(n, 11);
   });
 }
 

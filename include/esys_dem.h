@@ -243,7 +243,8 @@ int dem_set_stream(dem_sim* h, void* stream);
  * [6] interactions evaluated per step now, [7] threads per particle in use, [8] 1 when a neighbour
  * search is due at the head of the next step (a particle moved more than verletDist/2 since the
  * last search, dem_search_neighbors was called, or no step has run yet: what
- * TSubLattice::checkNeighbors reports, Parallel/SubLattice.hpp:2473-2520).  Returns entries written. */
+ * TSubLattice::checkNeighbors reports, Parallel/SubLattice.hpp:2473-2520), [9] launches of the multi-step kernel, [10] those of them that
+ * left early because a block's pruned lists did not fit it.  Returns entries written. */
 int dem_get_counters(dem_sim* h, long long* out, int n);
 
 /* Precision check of the FP32-force form, no reference counterpart: from the FP64 form, evaluates
