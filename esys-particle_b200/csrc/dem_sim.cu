@@ -1059,15 +1059,16 @@ struct DemSim {
     return ra.room >= 1024 && ra.pool >= ra.ppb / 4;
   }
 
-  // Lanes per particle of the single-step kernels when none is set.  Without bonds one lane: the
-  // multi-step kernel's order of summation, whichever of the two takes a call.  With bonds, a
-  // specimen with at least as many particles as the GPU keeps step threads resident (3 blocks of
-  // 256 per SM) already fills it at one lane per particle, and a smaller one spreads each
-  // particle's adjacency over lanes by its mean length.  The tiled kernels (kTiled) are chosen
+  // Lanes per particle of the single-step kernels when none is set.  A specimen with at least as many
+  // particles as the GPU keeps step threads resident (3 blocks of 256 per SM) already fills it at one
+  // lane per particle; a smaller one spreads each particle's adjacency over lanes by its mean length.
+  // dem_step takes one lane without bonds: the multi-step kernel's order of summation, whichever of the two
+  // takes a call.  A window has no multi-step form (40 steps forward of a frictional packing of 6,859: 707 us
+  // by the mean, 836 at one lane; of 64,000: 1232 and 1059).  The tiled kernels (kTiled) are chosen
   // explicitly or by the ensemble autotuner.
-  int pick_tpp() {
+  int pick_tpp(bool window = false) {
     if (tpp) return tpp == kTiled && !tiled_ok() ? 1 : tpp;
-    if (bond.empty() || n >= 768LL * sms()) return 1;
+    if ((bond.empty() && !window) || n >= 768LL * sms()) return 1;
     long long e = 0;
     for (auto& d : dyn) e += 2LL * d.second.m;
     for (auto& b : bond) e += 2LL * b.second.nb;
@@ -1361,7 +1362,7 @@ struct DemSim {
 
   int window_forward(int T, int K, double* R_host) {
     if (!win_begin(T, K)) return DEM_ERR_OVERFLOW;
-    const int t_pp = pick_tpp();
+    const int t_pp = pick_tpp(true);
     d_wall_partial.reserve((size_t)step_grid(n, t_pp) * kMaxWalls * 3);
     const bool two = split == 1;
     const long long cps = contacts_per_step();
@@ -1658,7 +1659,7 @@ struct DemSim {
                       double* gquat) {
     AdjArgs A = adj_begin(gR_host);
     const int K = win.K, T = win.T, nw = (int)wig.size();
-    const int t_pp = pick_tpp();
+    const int t_pp = pick_tpp(true);
     d_wall_partial.reserve((size_t)step_grid(n, t_pp) * kMaxWalls * 3);
     const bool two = split == 1;
     for (int c = win.nseg - 1; c >= 0; --c) {

@@ -403,3 +403,18 @@ def test_fitted_polydisperse_window_matches_dual_numbers(gpu, orc):
     gd = np.einsum("tgc,tgck->k", S.mse_grad(Rd, tgt), dR)
     layout = a.param_layout()
     _grad_vs(g["params"][[layout.index(k) for k in keys]], gd, 1e-4)
+
+
+def test_window_without_bonds_takes_lanes_by_the_mean(gpu):
+    """5.2 entries of the pair list a particle: two lanes (2.5 to 6), in the forward and its recompute."""
+    out = []
+    for lanes in (0, 2, 1):
+        s = S.friction_pack(gpu, nx=9, ny=6, nz=7, vscale=5.0)
+        s.set_option("threads_per_particle", lanes)
+        R = s.window_forward(40, 7)
+        out.append((s.particles(), s.window_adjoint(S.mse_grad(R, S.mse_target(R)))))
+    for k in ("pos", "vel", "angvel", "quat"):
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
+    assert np.array_equal(out[0][1]["params"], out[1][1]["params"])
+    assert not np.array_equal(out[0][0]["vel"], out[2][0]["vel"])  # one lane adds in another order
