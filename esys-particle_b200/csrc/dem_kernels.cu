@@ -802,14 +802,14 @@ void launch_place_cells(const Particles& P, const int* cell_start, const int* un
 }
 void launch_pairs_count(const Grid& g, const Particles& P, int cur, const int* cs, const int* cl, const ExclDev& ex,
                         int* count, cudaStream_t s) {
-  k_pairs_count<<<nblk((P.n + 1) * kSearchLanes, kSearchThreads), kSearchThreads, 0, s>>>(g, P, cur, cs, cl, ex, count);
+  k_pairs_count<<<nblk((P.n + 1LL) * kSearchLanes, kSearchThreads), kSearchThreads, 0, s>>>(g, P, cur, cs, cl, ex, count);
 }
 template <class H>
 void launch_pairs_write(const Grid& g, const Particles& P, int cur, const int* cs, const int* cl, const ExclDev& ex,
                         const int* start, unsigned long long* keys, int kind, const unsigned long long* old_keys,
                         int old_n, const int* old_p1, const H* old_hist, H* hist, cudaStream_t s) {
   if (P.n)
-    k_pairs_write<H><<<nblk(P.n * kSearchLanes, kSearchThreads), kSearchThreads, 0, s>>>(g, P, cur, cs, cl, ex, start, keys, kind, old_keys, old_n,
+    k_pairs_write<H><<<nblk((long long)P.n * kSearchLanes, kSearchThreads), kSearchThreads, 0, s>>>(g, P, cur, cs, cl, ex, start, keys, kind, old_keys, old_n,
                                                      old_p1, old_hist, hist);
 }
 template void launch_pairs_write<double4>(const Grid&, const Particles&, int, const int*, const int*, const ExclDev&,
