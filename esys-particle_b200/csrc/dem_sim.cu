@@ -1063,12 +1063,17 @@ struct DemSim {
   // particles as the GPU keeps step threads resident (3 blocks of 256 per SM) already fills it at one
   // lane per particle; a smaller one spreads each particle's adjacency over lanes by its mean length.
   // dem_step takes one lane without bonds: the multi-step kernel's order of summation, whichever of the two
-  // takes a call.  A window has no multi-step form (40 steps forward of a frictional packing of 6,859: 707 us
+  // takes a call, so that FP64 states do not depend on how the steps are dealt to calls.  In the FP32 form
+  // the two round unlike anyway, and up to kLanesFp32 particles per SM the mean decides (one step of a
+  // frictional packing of 13,824: 31 us, at one lane 41; of 32,768: 34 and 41; of 64,000: 45 and 42).
+  // A window has no multi-step form (40 steps forward of a frictional packing of 6,859: 707 us
   // by the mean, 836 at one lane; of 64,000: 1232 and 1059).  The tiled kernels (kTiled) are chosen
   // explicitly or by the ensemble autotuner.
+  static constexpr int kLanesFp32 = 256;
   int pick_tpp(bool window = false) {
     if (tpp) return tpp == kTiled && !tiled_ok() ? 1 : tpp;
-    if ((bond.empty() && !window) || n >= 768LL * sms()) return 1;
+    const bool by_mean = !bond.empty() || window || (fp32 && n < kLanesFp32 * (long long)sms());
+    if (!by_mean || n >= 768LL * sms()) return 1;
     long long e = 0;
     for (auto& d : dyn) e += 2LL * d.second.m;
     for (auto& b : bond) e += 2LL * b.second.nb;

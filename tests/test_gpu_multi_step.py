@@ -231,3 +231,21 @@ def test_short_calls(gpu, shape, squeeze, launches):
         assert a.counters()["launches"] - before == want, k
         b.step(k)
     _equal(a, b, ["friction"], ["floor", "roof"])
+
+
+@pytest.mark.parametrize("precision,lanes", [(64, 1), (32, 2)])
+def test_lanes_of_single_steps(gpu, precision, lanes):
+    """5.2 entries of the pair list a particle: one lane in FP64 (the states do not depend on how the steps
+    are dealt to calls), two by the mean in the FP32 form."""
+    a, b, c = (S.friction_pack(gpu, nx=9, ny=6, nz=7, vscale=5.0) for _ in range(3))
+    for s in (a, b, c):
+        s.set_option("precision", precision)
+    b.set_option("threads_per_particle", lanes)
+    for _ in range(20):
+        a.step(1)
+        b.step(1)
+    c.step(20)
+    pa, pb, pc = a.particles(), b.particles(), c.particles()
+    for k in ("pos", "vel", "angvel", "quat"):
+        assert np.array_equal(pa[k], pb[k]), k
+        assert precision == 32 or np.array_equal(pa[k], pc[k]), k
