@@ -137,15 +137,17 @@ def nrot_bonded_block_script(make, nx=5, ny=6, nz=5, dt=1e-4, k=1e4, rbreak=0.02
     return sim
 
 
-def friction_pack(make, nx=6, ny=5, nz=6, seed=2, periodic=False, dt=5e-5, vscale=0.5, squeeze=0.93):
+def friction_pack(make, nx=6, ny=5, nz=6, seed=2, periodic=False, dt=5e-5, vscale=0.5, squeeze=0.93, rad=None):
     """Small rotational frictional pack: slightly overlapping jittered lattice of
     RotSpheres (lognormal radii), RotFriction kn=ks=1e4 mu=0.6, elastic floor and
-    roof, random initial linear and angular velocities, linear + rotational damping."""
+    roof, random initial linear and angular velocities, linear + rotational damping.
+    ``rad`` replaces the drawn radii."""
     rng = np.random.default_rng(seed)
     g = np.stack(np.meshgrid(np.arange(nx), np.arange(ny), np.arange(nz), indexing="ij"), -1).reshape(-1, 3)
     spacing = 1.0 * squeeze
     pos = (g + 0.5) * spacing + rng.uniform(-0.03, 0.03, size=g.shape)
-    rad = np.clip(np.exp(np.log(0.5) + 0.25 * rng.standard_normal(len(g))) * 0.5 + 0.25, 0.3, 0.5)
+    drawn = np.clip(np.exp(np.log(0.5) + 0.25 * rng.standard_normal(len(g))) * 0.5 + 0.25, 0.3, 0.5)
+    rad = drawn if rad is None else rad
     n = len(g)
     Lx, Ly, Lz = nx * spacing, ny * spacing + 0.2, nz * spacing
     sim = make("RotSphere", 1.2, 0.2, (0, -0.1, 0), (Lx, Ly - 0.1, Lz), (1 if periodic else 0, 0, 0), dt)
