@@ -593,8 +593,8 @@ struct DemSim {
   // engine's latency for up to seven fields, one after another, was most of such a call.  Otherwise the
   // rows are packed on the device, then each wanted field is one copy into the caller's array
   // (direct DMA when the caller's memory is pinned).
-  // 8,000 rows take 99 us directly and 115 with the copies, 64,000 take 262 and 268; 125,000 and more
-  // are faster with the copies.
+  // Either precision form, us directly / with the copies: 512 rows 77 / 96, 4,096 90 / 107, 15,625 122 / 138,
+  // 32,768 174 / 185, 64,000 255 / 260; 125,000 and more are faster with the copies.
   static constexpr int kDirectRows = 1 << 16;
   int alive_n = -1;  // alive particles; -1: to be counted (only a neighbour search or a revival changes them)
   int get_particles(int* id, double* pos, double* vel, double* angvel, double* quat, double* force, double* moment) {
@@ -1047,9 +1047,10 @@ struct DemSim {
     // else the records stay in L2, and what is left is shared 60:40 between entries and results
     ra.one = 0;
     // A dense frictional packing in FP64 does not gain: nearly every listed pair touches, so pruning leaves
-    // the lists as long, and the law, evaluated for both owners, sets the pace of either kernel (40 steps of
-    // 64,000 particles with 5.8 entries each: 1333 us here, 1126 singly; 100 steps of 125,000 with 3.4:
-    // 1718 here, 2893 singly; in the FP32 form the former take 1018 and 1155).
+    // the lists as long, and the law, evaluated for both owners, sets the pace of either kernel.  40 steps of
+    // 74,000 particles here / singly, us: RotFriction at 4.2 entries each 536 / 853, at 5.2 918 / 870, at 5.95
+    // 1278 / 852; NRotFriction at 6.0 805 / 776 (RotSphere 1191 / 877); HertzMindlin at 6.0 1030 / 1004
+    // (RotSphere 1473 / 1112).  The FP32 form gains up to what fits (5.95 entries: 918 / 1036).
     if (!fp32 && fric && mean >= kRunDense) return false;
     const size_t fixed = run_layout(rot, fric, moment, fp32, false, ra.ppb, 0, 0).bytes + 128;
     if (ra.ppb > 65535 || fixed > kRunSmem / 2) return false;
