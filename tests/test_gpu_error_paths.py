@@ -68,6 +68,9 @@ def test_unknown_names_and_bad_arguments_leave_the_handle_usable(gpu):
     _arg_error(lambda: a.set_option("threads_per_particle", 3), "threads_per_particle")
     _arg_error(lambda: a.set_option("event_capacity", -1), "event_capacity")
     _arg_error(lambda: a.set_option("event_capacity", 2.5), "event_capacity")
+    for key in ("run_blocks", "barrier_polls"):
+        for v in (-1, 2.5, 2.0 ** 31, float("nan")):
+            _arg_error(lambda: a.set_option(key, v), key)
     _arg_error(lambda: a.step(-1), "negative step count")
     _arg_error(lambda: a.set_timestep(0.0), "time step")
     _arg_error(lambda: a.add_particles([0], [[1.0, 1.0, 1.0]], [0.4], [1.0]), "duplicate particle id")
